@@ -180,7 +180,8 @@ struct Params {
 };
 
 constexpr int kBBoxThreads = 512;
-constexpr int kTravThreads = 1024;
+constexpr int kTravThreads = 256;
+constexpr int kTravWarpsPerSm = 32;
 constexpr int kDispThreads = 512;
 
 // ---------------------------------------------------------------- kernels --

@@ -11,8 +11,11 @@
 #include <float.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "fa2_device.cuh"
 #include "fa2_learn.cuh"
+#include "fa2_walk.cuh"
 
 namespace fa2 {
 
@@ -143,12 +146,8 @@ __global__ void __launch_bounds__(1024) k_keys(int n, int tile, int first,
 
 // --------------------------------------------------------------- traverse --
 
-// Repulsion by a warp-cooperative preorder walk.  The 32 lanes of a warp
-// hold 32 consecutive bodies of the sorted order, as the reference's
-// ForceCalculationKernel does (src/RPBHKernels.cu:609-685); a cell is used as
-// a whole only if every lane passes d^2 + eps >= dq[level] (:661), else the
-// warp descends into it.  Bodies always interact.  The walk visits nodes in
-// the reference's order, so each lane adds the same terms in the same order.
+// Repulsion of every group of 32 consecutive sorted bodies, the reference's
+// warps (ForceCalculationKernel, src/RPBHKernels.cu:609-685), by walk_group.
 // The tail adds gravity + attraction, forms the swing and traction sums
 // (SpeedKernel, src/RPFA2Kernels.cu:111-202) and, in the last block to
 // finish, updates the adaptive speed (:204-219).
@@ -160,53 +159,41 @@ __global__ void __launch_bounds__(1024) k_keys(int n, int tile, int first,
 //
 // LEARN (the learned correction, fa2_learn.cuh) also records, per group, the
 // centroid and second moments of its bodies and the cells the whole group
-// accepted that are not small for their distance (a (group, node) pair,
-// gathered 32 at a time in registers, one per lane, and tested with
-// learn_keep when the 32 are written out), and
+// accepted that are not small for their distance (a (group, node) pair; the
+// lanes of a round that accepted a cell test it with learn_keep), and
 // writes each body's repulsion in sorted order instead of the tail: the MLP
 // and k_learn_tail finish the iteration.  The sums are the same.
 //
 // OVERLAP (prevent_overlap, with the monopole walk) repels accepted bodies by
 // the paper's anti-collision rule (overlap_factor) with the sizes of the
 // sorted bodies in ssize; a body node's sorted index is its owner's.
-template <bool QUAD, bool LEARN, bool OVERLAP = false>
-__global__ void __launch_bounds__(kTravThreads, 2048 / kTravThreads) k_traverse(
+template <bool QUAD, bool LEARN, bool OVERLAP, bool NORMAL_EPS>
+__global__ void __launch_bounds__(kTravThreads, kTravWarpsPerSm *kWarp / kTravThreads) k_traverse(
     int n, const float4 *__restrict nodes, const float2 *__restrict quad,
     const uint32_t *__restrict body_node,
     const uint32_t *__restrict vals, const float2 *__restrict fag,
     const float2 *__restrict fprev, float2 *__restrict f, float2 *__restrict warp_partial,
     DevState *st, IterCounters *ctr, Params prm, LearnBuffers lb,
-    const uint32_t *__restrict owner = nullptr, const float *__restrict ssize = nullptr) {
+    const uint32_t *__restrict owner, const float *__restrict ssize) {
+    __shared__ WalkWarp<QUAD, OVERLAP> s_walk[kTravThreads / kWarp];
     __shared__ float s_dq[64];
     __shared__ bool s_last;
     __shared__ float s_red[2][kTravThreads / kWarp];
     if (st->err || st->poison) return;
     if (threadIdx.x == 0) {
-        // src/RPBHKernels.cu:579-592: dq for the children of the root is
-        // (2 radius)^2 / theta^2 + eps, quartering per level.
-        float tmp = st->radius * 2;
-        float dq = tmp * tmp * prm.itolsq;
-        s_dq[0] = 0.0f;
-        for (int l = 1; l <= kLevels; ++l) {
-            s_dq[l] = dq + prm.epssq;
-            dq = dq * 0.25f;
-        }
-        for (int l = kLevels + 1; l < 64; ++l) s_dq[l] = 0.0f;
+        walk_thresholds(st->radius, prm, s_dq);
         if (blockIdx.x == 0) st->trav_radius = st->radius;
     }
     __syncthreads();
     const uint32_t end = st->tree_nodes;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nwarps = (n + 31) >> 5;
-    // Groups of 32 bodies are handed out one at a time from a global ticket:
-    // the work per group varies with the local density of the layout, and
-    // warps that take consecutive tickets walk neighbouring bodies, so the
-    // nodes they load are shared in L2.
-    for (;;) {
-        int w = 0;
-        if (lane == 0) w = (int)atomicAdd(&ctr->trav_ticket, 1u);
-        w = __shfl_sync(kFull, w, 0);
-        if (w >= nwarps) break;
+    // A warp's first group spreads the groups over the blocks (few groups: one
+    // per SM, not one SM's worth of warps on neighbouring groups); the others
+    // are handed out one at a time from a global ticket, because the work per
+    // group varies with the local density of the layout.
+    int w = wid * (int)gridDim.x + (int)blockIdx.x;
+    while (w < nwarps) {
         const int k = w * 32 + lane;
         const bool active = k < n;
         const float4 me = nodes[body_node[active ? k : n - 1]];
@@ -214,14 +201,7 @@ __global__ void __launch_bounds__(kTravThreads, 2048 / kTravThreads) k_traverse(
         // (unused) sums never feed anything
         const float px = active ? me.x : 1e30f, py = active ? me.y : 1e30f;
         const float my_size = OVERLAP && active ? ssize[k] : 0.0f;
-        // sum of m_j d / (d^2 + eps) over the accepted nodes; the body's own
-        // k_r m_i multiplies the sum once at the end
-        float ax = 0.0f, ay = 0.0f;
-        uint32_t node = 1;
-        // LEARN: the warp's accepted cells not yet written out; lane j holds
-        // the j-th of them
-        int npend = 0;
-        uint32_t my_cell = 0;
+        float gx = 0.0f, gy = 0.0f;
         if (LEARN) {
             // the group's centroid and second moments about it
             const float cnt = (float)__popc(__ballot_sync(kFull, active));
@@ -231,7 +211,8 @@ __global__ void __launch_bounds__(kTravThreads, 2048 / kTravThreads) k_traverse(
                 sx += __shfl_xor_sync(kFull, sx, o);
                 sy += __shfl_xor_sync(kFull, sy, o);
             }
-            const float gx = sx / cnt, gy = sy / cnt;
+            gx = sx / cnt;
+            gy = sy / cnt;
             const float u = active ? px - gx : 0.0f, v = active ? py - gy : 0.0f;
             float t0 = u * u + v * v, t1 = u * u - v * v, t2 = 2.0f * u * v;
 #pragma unroll
@@ -245,131 +226,59 @@ __global__ void __launch_bounds__(kTravThreads, 2048 / kTravThreads) k_traverse(
                 lb.ggeo[2 * w + 1] = make_float4(t1 / cnt, t2 / cnt, 0.0f, 0.0f);
             }
         }
-        // LEARN: the pending cells the group sees at a size ratio h / d of at
-        // least kLearnMinRatio theta (d from the group's centroid) to this
-        // warp's segment of the pair list, one atomic per flush
-        auto flush = [&]() {
-            __syncwarp();  // lane 0's store of the centroid is seen by all lanes
-            bool keep = false;
-            if (lane < npend) {
-                const float4 cell = __ldg(&nodes[my_cell]);
-                const float4 g0 = lb.ggeo[2 * w];
-                keep = learn_keep(s_dq[meta_level(__float_as_int(cell.w))], g0.x - cell.x,
-                                  g0.y - cell.y, prm.epssq);
-            }
+        // LEARN: a round's accepted cells that the group sees at a size ratio
+        // h / d of at least kLearnMinRatio theta (d from the group's centroid)
+        // go to this warp's segment of the pair list, one atomic per round
+        auto on_cells = [&](bool cell, const float4 &r, float thr, uint32_t node) {
+            const bool keep = cell && learn_keep(thr, gx - r.x, gy - r.y, prm.epssq);
             const unsigned km = __ballot_sync(kFull, keep);
+            if (km == 0) return;
             const unsigned nk = (unsigned)__popc(km);
-            const uint32_t seg = (blockIdx.x * (kTravThreads / kWarp) + (threadIdx.x >> 5)) %
+            const uint32_t seg = (blockIdx.x * (kTravThreads / kWarp) + (uint32_t)wid) %
                                  (uint32_t)kPairSegments;
             uint32_t base = 0;
-            if (lane == 0 && nk) base = atomicAdd(&ctr->pair_count[seg], nk);
+            if (lane == 0) base = atomicAdd(&ctr->pair_count[seg], nk);
             base = __shfl_sync(kFull, base, 0);
             const uint32_t idx = base + (uint32_t)__popc(km & ((1u << lane) - 1u));
             if (keep && idx < lb.seg_cap)
-                lb.pairs[(size_t)seg * lb.seg_cap + idx] = make_uint2((uint32_t)w, my_cell);
+                lb.pairs[(size_t)seg * lb.seg_cap + idx] = make_uint2((uint32_t)w, node);
             if (lane == 0 && base + nk > lb.seg_cap) atomicOr(&st->err, kErrPairs);
-            npend = 0;
         };
-        // An opened cell's first child is node + 1 and always exists, so only
-        // a jump to "next" can end the walk.
-        if (!QUAD && node < end) {
-            for (;;) {
-                const float4 r = __ldg(&nodes[node]);
-                const int meta = __float_as_int(r.w);
-                const float dx = px - r.x, dy = py - r.y;
-                const float d2 = sq_dist(dx, dy, prm.epssq);
-                // written as !(d2 < dq): a NaN distance accepts, so a warp
-                // with a non-finite lane still ends its walk
-                if (__all_sync(kFull, !(d2 < s_dq[meta_level(meta)]))) {
-                    float c;
-                    if (OVERLAP && meta_level(meta) == kBodyLevel)
-                        c = overlap_factor(d2, my_size, ssize[owner[node] >> 6], r.z);
-                    else
-                        c = __fdividef(r.z, d2);
-                    ax = fmaf(dx, c, ax);
-                    ay = fmaf(dy, c, ay);
-                    if (LEARN && meta_level(meta) != kBodyLevel) {
-                        if (lane == npend) my_cell = node;
-                        if (++npend == 32) flush();
-                    }
-                    node = meta_next(meta);
-                    if (node >= end) break;
-                } else {
-                    ++node;
-                }
-            }
-        }
-        if (QUAD && node < end) {
-            float4 r = __ldg(&nodes[node]);
-            for (;;) {
-                const int meta = __float_as_int(r.w);
-                const int lvl = meta_level(meta);
-                const float m = r.z;
-                const float dx = px - r.x, dy = py - r.y;
-                const float d2 = sq_dist(dx, dy, prm.epssq);
-                if (__all_sync(kFull, !(d2 < s_dq[lvl]))) {
-                    const uint32_t next = meta_next(meta);
-                    // the loads of the next node (and of this cell's second
-                    // moment) go out before this node's sums, so the warp
-                    // does not wait on them one after the other
-                    float2 q = make_float2(0.0f, 0.0f);
-                    if (lvl != kBodyLevel) q = __ldg(&quad[node]);
-                    if (next < end) r = __ldg(&nodes[next]);
-                    const float inv = __fdividef(1.0f, d2);
-                    const float c = m * inv;
-                    ax = fmaf(dx, c, ax);
-                    ay = fmaf(dy, c, ay);
-                    if (lvl != kBodyLevel) {
-                        // conj(a2) u^3 with u = 1 / conj(w) = w / |w|^2: |u| <= 1 / sqrt(eps)
-                        // and |a2 u^3| is below the monopole term's size, so nothing
-                        // overflows however far apart the bodies are
-                        const float ux = dx * inv, uy = dy * inv;
-                        const float xx = ux * ux, yy = uy * uy;
-                        const float ur = ux * fmaf(-3.0f, yy, xx);
-                        const float ui = uy * fmaf(-3.0f, xx, yy);
-                        ax = fmaf(q.x, ur, fmaf(-q.y, ui, ax));
-                        ay = fmaf(-q.x, ui, fmaf(-q.y, ur, ay));
-                        if (LEARN) {
-                            if (lane == npend) my_cell = node;
-                            if (++npend == 32) flush();
-                        }
-                    }
-                    node = next;
-                    if (node >= end) break;
-                } else {
-                    ++node;
-                    r = __ldg(&nodes[node]);
-                }
-            }
-        }
+        // sum of m_j d / (d^2 + eps) over the accepted nodes; the body's own
+        // k_r m_i multiplies the sum once at the end
+        const float2 a = walk_group<QUAD, OVERLAP, LEARN, NORMAL_EPS>(
+            s_walk[wid], s_dq, nodes, quad, owner, ssize, end, px, py, my_size, prm.epssq,
+            on_cells);
         // rounded on its own (never fused into the force sum that follows), so
         // the learned iteration, which stores it, adds the same value
         const float kmi = prm.k_r * me.z;
-        ax = __fmul_rn(ax, kmi);
-        ay = __fmul_rn(ay, kmi);
+        const float ax = __fmul_rn(a.x, kmi);
+        const float ay = __fmul_rn(a.y, kmi);
         if (LEARN) {
-            if (npend) flush();
             if (active) lb.rep[k] = make_float2(ax, ay);
-            continue;
-        }
-        float sw = 0.0f, tr = 0.0f;
-        if (active) {
-            const uint32_t i = vals[k];
-            const float2 g = fag[i], fp = fprev[i];
-            const float fx = g.x + ax, fy = g.y + ay;
-            f[i] = make_float2(fx, fy);
-            float dx = fx - fp.x, dy = fy - fp.y;
-            sw = me.z * sqrtf(sq_norm(dx, dy));
-            dx = fx + fp.x;
-            dy = fy + fp.y;
-            tr = me.z * (float)(sqrtf(sq_norm(dx, dy)) / 2.0);
-        }
+        } else {
+            float sw = 0.0f, tr = 0.0f;
+            if (active) {
+                const uint32_t i = vals[k];
+                const float2 g = fag[i], fp = fprev[i];
+                const float fx = g.x + ax, fy = g.y + ay;
+                f[i] = make_float2(fx, fy);
+                float dx = fx - fp.x, dy = fy - fp.y;
+                sw = me.z * sqrtf(sq_norm(dx, dy));
+                dx = fx + fp.x;
+                dy = fy + fp.y;
+                tr = me.z * (float)(sqrtf(sq_norm(dx, dy)) / 2.0);
+            }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            sw += __shfl_xor_sync(kFull, sw, o);
-            tr += __shfl_xor_sync(kFull, tr, o);
+            for (int o = 16; o > 0; o >>= 1) {
+                sw += __shfl_xor_sync(kFull, sw, o);
+                tr += __shfl_xor_sync(kFull, tr, o);
+            }
+            if (lane == 0) warp_partial[w] = make_float2(sw, tr);
         }
-        if (lane == 0) warp_partial[w] = make_float2(sw, tr);
+        if (lane == 0)
+            w = (int)(gridDim.x * (kTravThreads / kWarp) + atomicAdd(&ctr->trav_ticket, 1u));
+        w = __shfl_sync(kFull, w, 0);
     }
     if (LEARN) return;
     // last block: fixed-order sum of the per-warp partials, then the speed rule
@@ -900,36 +809,43 @@ void launch_keys(const Buffers &b, int nsm, cudaStream_t s) {
 
 
 
+namespace {
+
+// At most one block per group: the blocks past that would find no work.
+int traverse_grid(const Buffers &b, int nblocks) { return std::min(nblocks, (b.n + 31) / 32); }
+
+template <bool QUAD, bool LEARN, bool OVERLAP>
+void go_traverse(const Buffers &b, const Params &p, const LearnBuffers &lb, int nblocks,
+                 cudaStream_t s) {
+    auto go = [&](auto kernel) {
+        kernel<<<traverse_grid(b, nblocks), kTravThreads, 0, s>>>(
+            b.n, b.nodes, b.quad, b.body_node, b.vals[0], b.fag, b.fprev, b.f, b.warp_partial,
+            b.st, b.ctr, p, lb, b.owner, b.ssize);
+    };
+    if (p.epssq >= FLT_MIN)
+        go(k_traverse<QUAD, LEARN, OVERLAP, true>);
+    else
+        go(k_traverse<QUAD, LEARN, OVERLAP, false>);
+}
+
+}  // namespace
+
 void launch_traverse(const Buffers &b, const Params &p, int nblocks, cudaStream_t s) {
     const LearnBuffers none{};
-    auto go = [&](auto kernel) {
-        kernel<<<nblocks, kTravThreads, 0, s>>>(b.n, b.nodes, b.quad, b.body_node, b.vals[0],
-                                                b.fag, b.fprev, b.f, b.warp_partial, b.st, b.ctr,
-                                                p, none, nullptr, nullptr);
-    };
-    if (p.overlap) {
-        k_traverse<false, false, true><<<nblocks, kTravThreads, 0, s>>>(
-            b.n, b.nodes, b.quad, b.body_node, b.vals[0], b.fag, b.fprev, b.f, b.warp_partial,
-            b.st, b.ctr, p, none, b.owner, b.ssize);
-        return;
-    }
-    if (p.multipole >= 2)
-        go(k_traverse<true, false>);
+    if (p.overlap)
+        go_traverse<false, false, true>(b, p, none, nblocks, s);
+    else if (p.multipole >= 2)
+        go_traverse<true, false, false>(b, p, none, nblocks, s);
     else
-        go(k_traverse<false, false>);
+        go_traverse<false, false, false>(b, p, none, nblocks, s);
 }
 
 void launch_traverse_learn(const Buffers &b, const Params &p, const LearnBuffers &lb,
                            int nblocks, cudaStream_t s) {
-    auto go = [&](auto kernel) {
-        kernel<<<nblocks, kTravThreads, 0, s>>>(b.n, b.nodes, b.quad, b.body_node, b.vals[0],
-                                                b.fag, b.fprev, b.f, b.warp_partial, b.st, b.ctr,
-                                                p, lb, nullptr, nullptr);
-    };
     if (p.multipole >= 2)
-        go(k_traverse<true, true>);
+        go_traverse<true, true, false>(b, p, lb, nblocks, s);
     else
-        go(k_traverse<false, true>);
+        go_traverse<false, true, false>(b, p, lb, nblocks, s);
 }
 
 size_t guard_part_count(int ns) { return (size_t)ns * kGuardSplit; }
@@ -1004,18 +920,6 @@ void launch_sorted_ref_ids(int n, const uint32_t *ref_of, const uint32_t *vals, 
     k_sorted_ref_ids<<<grid_for(n, 256, 4096), 256, 0, s>>>(n, ref_of, vals, out);
 }
 
-int traverse_blocks_per_sm() {
-    // the walk lives on L1 hits: give L1 the most of the SM's on-chip memory
-    cudaFuncSetAttribute(k_traverse<false, false>, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
-    cudaFuncSetAttribute(k_traverse<true, false>, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
-    cudaFuncSetAttribute(k_traverse<false, false, true>,
-                         cudaFuncAttributePreferredSharedMemoryCarveout, 0);
-    // the learned walk keeps its pending pairs in registers, one per lane
-    cudaFuncSetAttribute(k_traverse<false, true>, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
-    cudaFuncSetAttribute(k_traverse<true, true>, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
-    int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_traverse<false, false>, kTravThreads, 0);
-    return nb < 1 ? 1 : nb;
-}
+int traverse_blocks_per_sm() { return kTravWarpsPerSm * kWarp / kTravThreads; }
 
 }  // namespace fa2

@@ -1,0 +1,63 @@
+"""The traversal at the sizes where its groups, lists and stacks have edges.
+
+The repulsion (fa2_repulsion_noalloc, which gives it alone) against the
+oracle's walk of the reference rule on the same positions.  The terms are the
+same set (the accept test is bit-exact); only their order of summation
+differs.  With T terms a body's float32 sum is off by at most T 2^-24 of the
+sum of the terms' magnitudes: under 1e-4 for T <= 1500, the suite's bar
+(relative RMSE).  The engine's cell centres are exact sums rounded once and the
+oracle's are float sums, so they differ by an ulp of the coordinate; the
+positions keep that far below the distances (the dense cluster sits at the
+origin, where an ulp is small), and no two coincide.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import rel_rmse
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-4
+
+
+def _positions(kind, n, seed):
+    rng = np.random.default_rng(seed)
+    xy = rng.uniform(-1000, 1000, (n, 2))
+    if kind == "clustered":  # deep chains of one-child cells, groups far apart inside
+        half = rng.random(n) < 0.5
+        xy[half] = rng.normal(0, 0.02, (int(half.sum()), 2))
+    return xy.astype(np.float32)
+
+
+def _check(kind, n, theta, seed=3):
+    import torch
+    from gpugraphlayout_b200 import _native
+    from oracle import oracle as O
+    xy = _positions(kind, n, seed)
+    mass = np.full(n, 2.0 if n < 3 else 3.0, np.float32)
+    prm = _native.Params()
+    _native.lib().fa2_default_params(C.byref(prm))
+    prm.scale, prm.theta = 10.0, theta
+    d_xy, d_mass = torch.from_numpy(xy).cuda(), torch.from_numpy(mass).cuda()
+    out = torch.full((n, 2), float("nan"), device="cuda")
+    assert _native.lib().fa2_repulsion_noalloc(
+        C.c_void_p(d_xy.data_ptr()), C.c_void_p(d_mass.data_ptr()), n, C.byref(prm), None,
+        C.c_void_p(out.data_ptr())) == 0
+    itolsq = float(np.float32(1.0) / (np.float32(theta) * np.float32(theta)))
+    ref, overflow, _ = O.Tree(xy, mass).repulsion(10.0, itolsq=itolsq)
+    assert not overflow
+    assert rel_rmse(out.cpu().numpy(), np.asarray(ref).reshape(-1, 2)) <= TOL
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 31, 32, 33, 63, 64, 65, 97, 1000, 1500])
+def test_group_edges(n):
+    _check("uniform", n, 1.0)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "clustered"])
+@pytest.mark.parametrize("theta", [0.2, 0.6, 1.0, 2.0])
+def test_opening_angles(kind, theta):
+    """From nearly every cell opened (full lists and stacks) to few."""
+    _check(kind, 1201, theta)
