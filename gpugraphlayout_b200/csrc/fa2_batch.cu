@@ -24,6 +24,7 @@
 
 #include "../../include/fa2b200.h"
 #include "fa2_device.cuh"
+#include "fa2_walk.cuh"
 
 namespace fa2 {
 
@@ -97,10 +98,14 @@ __device__ __forceinline__ NodeSums shfl_up_sums(const NodeSums &v, int o) {
     return t;
 }
 
-// Shared memory of the batch kernel (static part; sort histograms included).
+// Shared memory of the batch kernel (dynamic: over 48 KB with 1024 threads).
+// The sort's histograms and the warps' walks take turns.
 template <int T>
 struct BatchSmem {
-    uint32_t whist[T / kWarp][256];
+    union {
+        uint32_t whist[T / kWarp][256];
+        WalkWarp<false, false> walk[T / kWarp];
+    };
     uint32_t qsum[4][256];
     uint32_t base[256];
     uint32_t coff[256];
@@ -534,15 +539,7 @@ __device__ void phase_traverse(const BatchArgs &A, uint32_t base, uint32_t n, ch
     float2 *gpart = slot_ptr<float2>(slot, A.L.gpart);
     const int lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        // src/RPBHKernels.cu:579-592
-        float tmp = S.radius * 2;
-        float dq = tmp * tmp * A.prm.itolsq;
-        S.dq[0] = 0.0f;
-        for (int l = 1; l <= kLevels; ++l) {
-            S.dq[l] = dq + A.prm.epssq;
-            dq = dq * 0.25f;
-        }
-        for (int l = kLevels + 1; l < 64; ++l) S.dq[l] = 0.0f;
+        walk_thresholds(S.radius, A.prm, S.dq);
         S.ticket = 0;
     }
     __syncthreads();
@@ -557,29 +554,16 @@ __device__ void phase_traverse(const BatchArgs &A, uint32_t base, uint32_t n, ch
         const bool active = k < (int)n;
         const float4 me = nodes[body_node[active ? k : (int)n - 1]];
         const float px = active ? me.x : 1e30f, py = active ? me.y : 1e30f;
-        float ax = 0.0f, ay = 0.0f;
-        uint32_t node = 1;
-        if (node < end) {
-            for (;;) {
-                const float4 r = nodes[node];
-                const int meta = __float_as_int(r.w);
-                const float dx = px - r.x, dy = py - r.y;
-                const float d2 = sq_dist(dx, dy, A.prm.epssq);
-                // !(d2 < dq): a NaN distance accepts, so the walk still ends
-                if (__all_sync(kFullMask, !(d2 < S.dq[meta_level(meta)]))) {
-                    const float c = __fdividef(r.z, d2);
-                    ax = fmaf(dx, c, ax);
-                    ay = fmaf(dy, c, ay);
-                    node = meta_next(meta);
-                    if (node >= end) break;
-                } else {
-                    ++node;
-                }
-            }
-        }
+        auto none = [](bool, const float4 &, float, uint32_t) {};
+        WalkWarp<false, false> &W = S.walk[threadIdx.x >> 5];
+        const float2 a =
+            A.prm.epssq >= FLT_MIN
+                ? walk_group<false, false, false, true>(W, S.dq, nodes, nullptr, nullptr, nullptr,
+                                                        end, px, py, 0.0f, A.prm.epssq, none)
+                : walk_group<false, false, false, false>(W, S.dq, nodes, nullptr, nullptr, nullptr,
+                                                         end, px, py, 0.0f, A.prm.epssq, none);
         const float kmi = A.prm.k_r * me.z;
-        ax *= kmi;
-        ay *= kmi;
+        const float ax = __fmul_rn(a.x, kmi), ay = __fmul_rn(a.y, kmi);
         float sw = 0.0f, tr = 0.0f;
         if (active) {
             const uint32_t i = vals[k];
@@ -642,15 +626,16 @@ __device__ void phase_displace(const BatchArgs &A, uint32_t base, uint32_t n, ch
     __syncthreads();
 }
 
-// 2048 threads per SM: 32 registers a thread, which spills about 1.4 KB of
-// the tree and sort phases' state to local memory (L1).  The walk, like the
-// single-graph engine's, needs every warp the SM holds to cover its load
-// latency: on the 4096-graph batch this bound gives 124 batch iterations/s
-// against 107 with 64 registers and 1024 threads per SM (118 with 42
-// registers and 1536 threads).
+// 1024 threads per SM, 64 registers a thread: a warp's walk has 32 loads in
+// flight, so it needs few warps, and at 32 registers it spills.  Measured on 512
+// graphs of 50 to 20,000 nodes (512-thread CTAs up to 4096 nodes, 1024-thread
+// CTAs above), 1024, 1536 and 2048 threads per SM: 1.74, 1.74 and 1.99 ms an
+// iteration; on 96 graphs of 50 to 600 nodes 90, 103 and 112 us.
+constexpr int kBatchThreadsPerSm = 1024;
 template <int T, bool LINLOG>
-__global__ void __launch_bounds__(T, 2048 / T) k_batch(BatchArgs A) {
-    __shared__ BatchSmem<T> S;
+__global__ void __launch_bounds__(T, kBatchThreadsPerSm / T) k_batch(BatchArgs A) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    BatchSmem<T> &S = *reinterpret_cast<BatchSmem<T> *>(smem_raw);
     char *slot = A.slots + (size_t)blockIdx.x * A.L.bytes;
     float2 *fa = slot_ptr<float2>(slot, A.L.fa);
     for (;;) {
@@ -833,8 +818,11 @@ void bfree(fa2_batch *b) {
 template <int T>
 int occupancy() {
     int a = 0, c = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_batch<T, false>, T, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_batch<T, true>, T, 0);
+    const int bytes = (int)sizeof(BatchSmem<T>);
+    cudaFuncSetAttribute(k_batch<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(k_batch<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_batch<T, false>, T, bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_batch<T, true>, T, bytes);
     return std::max(1, std::min(a, c));
 }
 
@@ -893,9 +881,9 @@ int configure(fa2_batch *b, uint32_t split, int small_threads, int large_threads
 template <bool LINLOG>
 void launch_class(const BatchClass &c, cudaStream_t s) {
     switch (c.threads) {
-        case 256: k_batch<256, LINLOG><<<c.grid, 256, 0, s>>>(c.args); break;
-        case 512: k_batch<512, LINLOG><<<c.grid, 512, 0, s>>>(c.args); break;
-        default: k_batch<1024, LINLOG><<<c.grid, 1024, 0, s>>>(c.args); break;
+        case 256: k_batch<256, LINLOG><<<c.grid, 256, sizeof(BatchSmem<256>), s>>>(c.args); break;
+        case 512: k_batch<512, LINLOG><<<c.grid, 512, sizeof(BatchSmem<512>), s>>>(c.args); break;
+        default: k_batch<1024, LINLOG><<<c.grid, 1024, sizeof(BatchSmem<1024>), s>>>(c.args); break;
     }
 }
 

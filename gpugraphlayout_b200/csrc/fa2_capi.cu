@@ -27,11 +27,12 @@ using namespace fa2;
 
 namespace {
 
-constexpr int kNumSlots = 10;
+constexpr int kNumSlots = 11;
 const char *const kSlotNames[kNumSlots] = {"attract",  "keys",     "sort",    "tree_count",
                                            "emit",     "traverse", "displace", "moments",
-                                           "quadrupole", "learn"};
-enum Slot { S_ATTRACT, S_KEYS, S_SORT, S_COUNT, S_EMIT, S_TRAV, S_DISP, S_MOM, S_QUAD, S_LEARN };
+                                           "quadrupole", "learn",    "tree"};
+// the tree build is one kernel ("tree"); the slots of its phases stay empty
+enum Slot { S_ATTRACT, S_TRAV = 5, S_DISP, S_MOM, S_QUAD, S_LEARN, S_TREE };
 
 // The last CUDA error a call of this thread met, with the source line that saw
 // it (fa2_last_cuda_error).
@@ -58,11 +59,11 @@ struct fa2_ctx {
     size_t scratch_bytes = 0;
     float2 *stage_xy = nullptr;    // n, reference order
     DevState *h_state = nullptr;   // pinned: the state after fa2_step_host's iterations
-    int *h_iters = nullptr;        // pinned: iterations done before them
+    int *h_before = nullptr;       // pinned: iters_done and resorts before them
     uint32_t *stage_ids = nullptr; // n
     int bbox_blocks = 0, trav_blocks = 0;
     cudaStream_t sA = nullptr, sB = nullptr;
-    cudaEvent_t evFork = nullptr, evJoin = nullptr, evCounted = nullptr;
+    cudaEvent_t evFork = nullptr, evJoin = nullptr;
     cudaEvent_t evEmitted = nullptr, evA2 = nullptr;  // the learned cells' a2 pass on stream B
     // graphs
     cudaGraphExec_t exec = nullptr;
@@ -72,6 +73,7 @@ struct fa2_ctx {
     std::vector<cudaEvent_t> slot_events;      // events captured into the timed graph
     std::vector<cudaEvent_t> event_pool;       // per (iteration, slot, start/end)
     int last_perturb_rounds = 0;
+    int resorts_before = 0;  // DevState::resorts when the last step call began
     bool overlap = true;  // attraction on stream B beside the tree build
     // accuracy guard (fa2_set_accuracy_guard)
     int guard_every = 0, guard_samples = 0, guard_cap = 0, guard_left = 0;
@@ -168,13 +170,12 @@ void free_all(fa2_ctx *c) {
     c->allocs.clear();
     if (c->evFork) cudaEventDestroy(c->evFork);
     if (c->evJoin) cudaEventDestroy(c->evJoin);
-    if (c->evCounted) cudaEventDestroy(c->evCounted);
     if (c->evEmitted) cudaEventDestroy(c->evEmitted);
     if (c->evA2) cudaEventDestroy(c->evA2);
     if (c->sA) cudaStreamDestroy(c->sA);
     if (c->sB) cudaStreamDestroy(c->sB);
     if (c->h_state) cudaFreeHost(c->h_state);
-    if (c->h_iters) cudaFreeHost(c->h_iters);
+    if (c->h_before) cudaFreeHost(c->h_before);
 }
 
 // Nodes in degree-descending order (ties by reference id), a symmetric CSR
@@ -299,35 +300,19 @@ void enqueue_iteration(fa2_ctx *c, bool full, bool perturb_first, bool timed) {
         mark(S_ATTRACT, 0, B);
         launch_attract(b, c->kp, c->plan, B);
         mark(S_ATTRACT, 1, B);
-        if (!quad) cudaEventRecord(c->evJoin, B);
+        cudaEventRecord(c->evJoin, B);
     }
     if (perturb_first) launch_runs(b, 1, c->nsm, A);
-    mark(S_KEYS, 0, A);
-    launch_keys(b, c->nsm, A);
-    mark(S_KEYS, 1, A);
-    mark(S_SORT, 0, A);
-    launch_sort(b, A);
-    launch_fix_low(b, c->nsm, A);
-    mark(S_SORT, 1, A);
-    mark(S_COUNT, 0, A);
-    launch_tree_count(b, quad, A);
-    mark(S_COUNT, 1, A);
-    // The tree count leaves the sorted bodies' grid offsets and masses for the
-    // moment scan; with stream B in use the scan runs there, beside the emit.
+    mark(S_TREE, 0, A);
+    launch_build(b, quad, c->nsm, A);
+    mark(S_TREE, 1, A);
+    // the build leaves the sorted bodies' grid offsets and masses for the
+    // moment scan
     if (quad) {
-        cudaStream_t M = side ? B : A;
-        if (side) {
-            cudaEventRecord(c->evCounted, A);
-            cudaStreamWaitEvent(B, c->evCounted, 0);
-        }
-        mark(S_MOM, 0, M);
-        launch_moments(b, M);
-        mark(S_MOM, 1, M);
-        if (side) cudaEventRecord(c->evJoin, B);
+        mark(S_MOM, 0, A);
+        launch_moments(b, A);
+        mark(S_MOM, 1, A);
     }
-    mark(S_EMIT, 0, A);
-    launch_emit(b, c->nsm, A);
-    mark(S_EMIT, 1, A);
     if (learn) {
         // the cells' second moments (a feature of the pairs), beside the walk
         // on stream B when it is in use; the MLP waits for them
@@ -456,36 +441,24 @@ int resolve_poison(fa2_ctx *c, DevState *st) {
     int rounds = 0;
     while (st->poison) {
         if (++rounds > kMaxReplayRounds) return FA2_ERR_DEVICE_LIMIT;
-        // A run of keys equal in the sorted digits was too long for
-        // k_fix_low: the iteration again, sorted on every digit.  Otherwise
-        // coincident bodies: the iteration again after the .99 scaling.
-        const bool resort = st->resort != 0;
-        if (resort) {
-            c->b.sort_first = 0;
-            drop_graphs(c);
-            CK(cudaMemsetAsync(&c->b.st->resort, 0, sizeof(int), c->sA));
-        }
+        // coincident bodies: the iteration again after the .99 scaling
         CK(cudaMemsetAsync(&c->b.st->poison, 0, sizeof(int), c->sA));
-        enqueue_iteration(c, false, !resort, false);
+        enqueue_iteration(c, false, true, false);
         CK(cudaGetLastError());
         int s = read_state(c, st);
         if (s) return s;
         if (st->err) return FA2_ERR_DEVICE_LIMIT;
     }
-    c->last_perturb_rounds = rounds;
+    c->last_perturb_rounds += rounds;
     return FA2_OK;
 }
 
-// After a tree no deeper than kShallowLevel (kMidLevel) the next sorts skip
-// their two lowest digits (their lowest one); k_fix_low keeps the order
-// exact.  The choice is part of the captured graphs, which are dropped when
-// it changes.
+// The digits the last tree's depth lets the next sorts leave to the fix-up:
+// the two lowest after a tree no deeper than kShallowLevel, the lowest one
+// after one no deeper than kMidLevel (fa2_stats.sort_passes).
 void choose_sort_passes(fa2_ctx *c, const DevState &st) {
     const int l = st.max_level;
-    const int first = l <= 0 ? 0 : (l <= kShallowLevel ? 2 : (l <= kMidLevel ? 1 : 0));
-    if (first == c->b.sort_first) return;
-    c->b.sort_first = first;
-    drop_graphs(c);
+    c->b.sort_first = l <= 0 ? 0 : (l <= kShallowLevel ? 2 : (l <= kMidLevel ? 1 : 0));
 }
 
 // Runs n iterations; with `timed`, kernel_sum accumulates per-slot device ms.
@@ -498,6 +471,7 @@ int run_steps(fa2_ctx *c, int32_t n_iters, bool timed, std::vector<double> *kern
     if (s) return s;
     int done = 0;
     c->last_perturb_rounds = 0;
+    c->resorts_before = st.resorts;
     while (done < n_iters) {
         choose_sort_passes(c, st);
         // (re)captured here: a guard fallback drops the graphs
@@ -803,6 +777,7 @@ fa2_ctx *fa2_create(const fa2_graph_desc *g, const fa2_params *prm, int *status)
     uint64_t cap = std::min<uint64_t>(33ull * n + 64, kMaxTreeNodes);
     b.capacity = (uint32_t)cap;
     uint32_t *d_off = nullptr, *d_ref = nullptr;
+    char *totals = nullptr;
     int4 *d_col = nullptr;
     float4 *d_w = nullptr;
     int s = FA2_OK;
@@ -811,12 +786,16 @@ fa2_ctx *fa2_create(const fa2_graph_desc *g, const fa2_params *prm, int *status)
         (s = dalloc(c, &d_off, (size_t)n + 1)) || (s = dalloc(c, &d_col, col.size() / 4)) ||
         (s = dalloc(c, &d_ref, n)) || (s = dalloc(c, &b.keys[0], n)) ||
         (s = dalloc(c, &b.keys[1], n)) || (s = dalloc(c, &b.vals[0], n)) ||
-        (s = dalloc(c, &b.vals[1], n)) || (s = dalloc(c, &b.lcp, n)) ||
+        (s = dalloc(c, &b.vals[1], n)) || (s = dalloc(c, &b.lcp, pad64(n))) ||
+        (s = dalloc(c, &b.sbody, n)) || (s = dalloc(c, &b.rowmin, pad64(((size_t)n + 31) / 32))) ||
+        (s = dalloc(c, &b.tilemin, pad64((size_t)c->nsm))) ||
+        (s = dalloc(c, &b.defer, ((size_t)n + 31) / 32 * (kLevels + 1))) ||
         (s = dalloc(c, &b.group, n)) || (s = dalloc(c, &b.body_node, n)) ||
         (s = dalloc(c, &b.nodes, cap + 1)) ||  // + one spare slot
         (s = dalloc(c, &b.owner, cap)) ||
         (s = dalloc(c, &b.pm, (size_t)n + 1)) || (s = dalloc(c, &b.pxy, 2 * ((size_t)n + 1))) ||
-        (s = dalloc(c, &b.lookback, (size_t)count_tiles((int)n))) ||
+        (s = dalloc(c, &b.sort_counts, build_counts(build_blocks((int)n, c->nsm)))) ||
+        (s = dalloc(c, &totals, build_totals_bytes(build_blocks((int)n, c->nsm)))) ||
         (s = dalloc(c, &b.warp_partial, (n + 31) / 32)) ||
         (s = dalloc(c, &b.st, 1)) || (s = dalloc(c, &c->stage_xy, n)) ||
         (s = dalloc(c, &c->stage_ids, n)))
@@ -831,20 +810,15 @@ fa2_ctx *fa2_create(const fa2_graph_desc *g, const fa2_params *prm, int *status)
     b.csr_col4 = d_col;
     b.csr_w4 = d_w;
     b.ref_of = d_ref;
-    // one memset clears counters, histograms, per-tile digit counts and the
-    // tree-count look-back flags
-    b.sort_rounds = sort_rounds((int)n, c->nsm);
-    const size_t sort_counts = (size_t)8 * sort_tiles_max((int)n) * 256;
-    const size_t count_status = (size_t)count_tiles((int)n);
+    b.build_totals = totals;
+    // one memset clears the counters and the moment scan's look-back flags
     const size_t mom_status = (size_t)mom_tiles((int)n);
-    c->scratch_bytes = sizeof(IterCounters) + 4 * (sort_counts + count_status + mom_status);
+    c->scratch_bytes = sizeof(IterCounters) + 4 * mom_status;
     char *scr = nullptr;
     if ((s = dalloc(c, &scr, c->scratch_bytes))) return fail(s);
     c->scratch = scr;
     b.ctr = (IterCounters *)scr;
-    b.sort_counts = (uint32_t *)(scr + sizeof(IterCounters));
-    b.count_status = b.sort_counts + sort_counts;
-    b.mom_status = b.count_status + count_status;
+    b.mom_status = (uint32_t *)(scr + sizeof(IterCounters));
 
     // The tree chain (stream A) is the critical path; the attraction (stream B)
     // only has to finish before the traversal.  With A at the higher priority
@@ -856,16 +830,15 @@ fa2_ctx *fa2_create(const fa2_graph_desc *g, const fa2_params *prm, int *status)
         cudaStreamCreateWithPriority(&c->sB, cudaStreamNonBlocking, prio_low) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->evFork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->evJoin, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->evCounted, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->evEmitted, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->evA2, cudaEventDisableTiming) != cudaSuccess ||
         cudaMallocHost(&c->h_state, sizeof(DevState)) != cudaSuccess ||
-        cudaMallocHost(&c->h_iters, sizeof(int)) != cudaSuccess)
+        cudaMallocHost(&c->h_before, 2 * sizeof(int)) != cudaSuccess)
         return fail(FA2_ERR_CUDA);
     c->slot_events.resize(kNumSlots * 2);
     for (auto &e : c->slot_events)
         if (cudaEventCreate(&e) != cudaSuccess) return fail(FA2_ERR_CUDA);
-    sort_set_smem_attr();
+    build_set_smem_attr();
     c->trav_blocks = c->nsm * traverse_blocks_per_sm();
 
     cudaStream_t A = c->sA;
@@ -955,7 +928,10 @@ int fa2_step_host(fa2_ctx *c, const float *xy_in, int32_t n_iters, float *xy_out
         CK(cudaMemsetAsync(&c->b.st->err, 0, sizeof(int), A));
         launch_bbox(c->b, c->bbox_blocks, A);
     }
-    CK(cudaMemcpyAsync(c->h_iters, &c->b.st->iters_done, sizeof(int), cudaMemcpyDeviceToHost, A));
+    static_assert(offsetof(DevState, resorts) == offsetof(DevState, iters_done) + sizeof(int),
+                  "iters_done and resorts are read with one copy");
+    CK(cudaMemcpyAsync(c->h_before, &c->b.st->iters_done, 2 * sizeof(int),
+                       cudaMemcpyDeviceToHost, A));
     c->last_perturb_rounds = 0;
     for (int it = 0; it < n_iters; ++it) CK(cudaGraphLaunch(c->exec, A));
     CK(cudaMemcpyAsync(c->h_state, c->b.st, sizeof(DevState), cudaMemcpyDeviceToHost, A));
@@ -966,15 +942,15 @@ int fa2_step_host(fa2_ctx *c, const float *xy_in, int32_t n_iters, float *xy_out
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(A));
     DevState st = *c->h_state;
+    c->resorts_before = c->h_before[1];
     if (st.err) return FA2_ERR_DEVICE_LIMIT;
-    int completed = st.iters_done - *c->h_iters;
+    int completed = st.iters_done - c->h_before[0];
     if (completed == n_iters && !st.poison) {
         choose_sort_passes(c, st);
         return FA2_OK;
     }
-    // An iteration was replayed (coincident bodies, or a sort that needs all
-    // its digits): the iterations after it did nothing.  The rest as
-    // fa2_step does it, then the positions again.
+    // An iteration needs a replay (coincident bodies): the iterations after it
+    // did nothing.  The rest as fa2_step does it, then the positions again.
     if (st.poison) {
         if ((s = resolve_poison(c, &st))) return s;
         completed += 1;
@@ -1030,7 +1006,7 @@ int fa2_get_stats(fa2_ctx *c, fa2_stats *out) {
     out->tree_nodes = st.tree_nodes;
     out->tree_cells = st.tree_nodes >= c->n ? st.tree_nodes - c->n : 0;
     out->max_level = st.max_level;
-    out->perturb_rounds = c->last_perturb_rounds;
+    out->perturb_rounds = c->last_perturb_rounds + (c->n ? st.resorts - c->resorts_before : 0);
     out->device_error = st.err;
     out->nnz_padded = c->nnz_pad;
     out->global_speed = st.global_speed;
@@ -1448,15 +1424,11 @@ int fa2_learn_collect(fa2_learn_set *set, fa2_ctx *c, float theta, int32_t multi
     kp.itolsq = 1.0f / (theta * theta);
     kp.multipole = multipole;
     Buffers b = c->b;
-    b.sort_first = 0;  // every digit: the walk needs no earlier tree
     cudaStream_t A = c->sA;
     CK(cudaMemsetAsync(c->scratch, 0, c->scratch_bytes, A));
     CK(cudaMemsetAsync(set->st_count, 0, sizeof(unsigned long long), A));
-    launch_keys(b, c->nsm, A);
-    launch_sort(b, A);
-    launch_tree_count(b, multipole >= 2, A);
+    launch_build(b, multipole >= 2, c->nsm, A);
     if (multipole >= 2) launch_moments(b, A);
-    launch_emit(b, c->nsm, A);
     if (multipole >= 2) launch_quad_cells(b, c->nsm, A);
     launch_cell_a2(b, c->lb, c->nsm, A);
     launch_traverse_learn(b, kp, c->lb, c->trav_blocks, A);

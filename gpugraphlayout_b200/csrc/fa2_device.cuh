@@ -54,30 +54,42 @@ __device__ __forceinline__ float overlap_factor(float d2, float si, float sj, fl
 
 // --------------------------------------------------- shared by the kernels --
 
+// Spreads the bits of v to the even bits of the result.
+__device__ __forceinline__ uint64_t spread_bits(uint32_t v) {
+    uint64_t x = v;
+    x = (x | (x << 16)) & 0x0000FFFF0000FFFFull;
+    x = (x | (x << 8)) & 0x00FF00FF00FF00FFull;
+    x = (x | (x << 4)) & 0x0F0F0F0F0F0F0F0Full;
+    x = (x | (x << 2)) & 0x3333333333333333ull;
+    return (x | (x << 1)) & 0x5555555555555555ull;
+}
+
 // Quadrant digits of (px, py) under the root cell, computed the way
 // TreeBuildingKernel walks down (src/RPBHKernels.cu:217-241): the child
 // centre is the parent centre +/- r, r halving per level; a coordinate
-// equal to the centre goes to the low side.
+// equal to the centre goes to the low side.  Bit x of a digit is x < px, which
+// is the sign of x - px (a difference of unequal floats is never zero, and
+// with -0 turned into +0 at the start no zero difference is negative): four
+// instructions per coordinate and level, the two coordinates' bits apart
+// until the end.
 __device__ __forceinline__ uint64_t morton_key(float px, float py, float x, float y, float r) {
-    uint64_t key = 0;
+    uint32_t bx = 0, by = 0;
+    px += 0.0f;
+    py += 0.0f;
+    x += 0.0f;
+    y += 0.0f;
 #pragma unroll 8
     for (int lvl = 0; lvl < kLevels; ++lvl) {
         r *= 0.5f;
-        int j = 0;
-        float dx = -r, dy = -r;
-        if (x < px) {
-            j = 1;
-            dx = r;
-        }
-        if (y < py) {
-            j |= 2;
-            dy = r;
-        }
-        x = __fadd_rn(x, dx);
-        y = __fadd_rn(y, dy);
-        key = (key << 2) | (uint64_t)j;
+        const uint32_t ri = __float_as_uint(r);
+        const uint32_t tx = __float_as_uint(__fadd_rn(x, -px));
+        const uint32_t ty = __float_as_uint(__fadd_rn(y, -py));
+        x = __fadd_rn(x, __uint_as_float(ri | (~tx & 0x80000000u)));
+        y = __fadd_rn(y, __uint_as_float(ri | (~ty & 0x80000000u)));
+        bx = __funnelshift_l(tx, bx, 1);
+        by = __funnelshift_l(ty, by, 1);
     }
-    return key;
+    return spread_bits(bx) | (spread_bits(by) << 1);
 }
 
 

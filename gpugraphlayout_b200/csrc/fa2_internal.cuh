@@ -1,8 +1,8 @@
 // fa2_internal.cuh -- device data layout and kernel entry points of the B200
 // ForceAtlas2 engine.  Host code in fa2_capi.cu enqueues one iteration as
 //
-//   stream A: keys -> sort (8 passes) -> tree_count -> emit -> [join B]
-//             -> traverse (+ speed) -> displace (+ next bounding box)
+//   stream A: build (the quadtree) -> [join B] -> traverse (+ speed)
+//             -> displace (+ next bounding box)
 //   stream B: attract (gravity + attraction)
 //
 // which replaces the eleven launches of CUDAForceAtlas2::doStep
@@ -24,7 +24,7 @@ constexpr int kDeepLevels = 64;    // levels past 32 used to order such a run
 
 // Device error bits (DevState::err).  Any of them stops the iteration.
 enum : int {
-    kErrScanWait = 2,      // a tree-count tile waited too long
+    kErrScanWait = 2,      // a block of the tree build or the moment scan waited too long
     kErrRunTooLong = 4,    // more than kMaxRun bodies share a 64-bit key
     kErrTreeTooLarge = 8,  // the quadtree needs more nodes than allocated
     kErrNonFinite = 16,    // a position is NaN or infinite
@@ -39,54 +39,38 @@ struct DevState {
     int poison;          // coincident bodies seen: this iteration is replayed
     int err;             // kErr* bits
     int iters_done;      // completed iterations
+    int resorts;         // sorts done again on every digit (read with iters_done)
     uint32_t tree_nodes; // nodes of the last quadtree
     int max_level;
     float swg_sum, etra_sum;
     unsigned long long interactions;  // body-node force terms of the last traversal
     unsigned long long visits;        // body-node acceptance tests of the last traversal
     float trav_radius;                // root radius the last traversal used
-    int resort;                       // a sort that skipped low digits needs all of them
+    int resort;                       // this sort skipped low digits that it needs
+    int deep;                         // bodies that share a whole 64-bit key
+    int cells[5];                     // largest cell of the last tree at levels 12, 16, .., 28
 };
 
 // Per-iteration scratch, cleared by one memset at the start of an iteration.
 struct IterCounters {
     unsigned bbox_done;
-    unsigned sort_ticket[8];
-    unsigned count_ticket;
+    unsigned build_bar;  // barrier arrivals of the tree build
     unsigned trav_ticket;
     unsigned trav_done;
     unsigned disp_done;
     unsigned mom_ticket;
-    unsigned pad[1];
+    unsigned pad[2];
     unsigned pair_count[16];  // (group, cell) pairs of a learned walk, per pair segment
-    unsigned hist[8][256];  // per-pass digit histograms of the sort keys
 };
 
-// Sort geometry: one tile per block, kSortThreads threads holding `rounds`
-// keys each.  The rounds (4, 5 or 6) are chosen per context so that, where
-// possible, every tile gets an SM of its own (see sort_rounds).
-constexpr int kSortThreads = 1024;
-constexpr int kSortWarps = kSortThreads / kWarp;
-constexpr int kSortMinRounds = 4;
-constexpr int kSortMaxRounds = 6;
-constexpr int kSortTileMin = kSortThreads * kSortMinRounds;  // 4096 keys
-constexpr int kCountThreads = 256;
-constexpr int kCountItems = 4;
-constexpr int kCountTile = kCountThreads * kCountItems;  // 1024 bodies
-
-inline int sort_tiles(int n, int rounds) {
-    const int tile = kSortThreads * rounds;
-    return (n + tile - 1) / tile;
+// Blocks of the tree build: 512 bodies or more each, at most one per SM.
+constexpr int kBuildMinTile = 512;
+inline int build_blocks(int n, int nsm) {
+    const int b = (n + kBuildMinTile - 1) / kBuildMinTile;
+    return b < 1 ? 1 : (b > nsm ? nsm : b);
 }
-// Upper bound on the tiles of any rounds choice (for sizing buffers).
-inline int sort_tiles_max(int n) { return sort_tiles(n, kSortMinRounds); }
-// The fewest rounds that give no more tiles than SMs; past that, the minimum.
-inline int sort_rounds(int n, int nsm) {
-    for (int r = kSortMinRounds; r <= kSortMaxRounds; ++r)
-        if (sort_tiles(n, r) <= nsm) return r;
-    return kSortMinRounds;
-}
-inline int count_tiles(int n) { return (n + kCountTile - 1) / kCountTile; }
+// Digit counts of the sort passes: [8][blocks][256].
+inline size_t build_counts(int blocks) { return (size_t)8 * blocks * 256; }
 
 // Moment scan (quadrupole option): bodies per tile and tiles.
 constexpr int kMomThreads = 256;
@@ -106,13 +90,6 @@ struct AttractPlan {
     AttractBucket b[kMaxBuckets];
     int nbuckets;
     int nblocks;
-};
-
-// Tile sums of k_tree_count's single-pass scan (written before the tile's
-// flag word is set; see fa2_tree.cu).
-struct LookbackSums {
-    long long agg_m, incl_m;
-    __int128 agg_x, agg_y, incl_x, incl_y;
 };
 
 // Exact moments of a run of sorted bodies on the fixed-point grid of 2^-44
@@ -142,7 +119,11 @@ struct Buffers {
     uint64_t *keys[2];
     uint32_t *vals[2];
     // tree
-    int8_t *lcp;              // n
+    float4 *sbody;            // n: sorted bodies, x, y, mass, id
+    uint8_t *lcp;             // n, padded to 64: digits shared with the next sorted body, + 1
+    uint8_t *rowmin;          // rows of 32 bodies, padded to 64: the least of lcp
+    uint8_t *tilemin;         // tree-build tiles, padded to 64: the least of lcp
+    uint32_t *defer;          // 33 per row: the tree build's cells that end in a later row
     uint32_t *group;          // n: first preorder node of body k's group
     uint32_t *body_node;      // n: preorder node of sorted body k
     uint32_t *owner;          // capacity: per node, sorted body k << 6 | cell offset (63: body)
@@ -156,16 +137,14 @@ struct Buffers {
     uint32_t capacity;
     long long *pm;            // n + 1: exclusive prefix of mass over sorted bodies
     __int128 *pxy;            // 2(n + 1): prefix of mass x fixed-point offset, x and y
-    LookbackSums *lookback;   // count tiles: tile sums of the tree-count scan
+    void *build_totals;       // tree-build blocks: their tiles' sums (NodeSums)
     // reductions
     float4 *bbox_partial;     // bbox blocks
     float2 *warp_partial;     // one per 32 sorted bodies
     DevState *st;
     IterCounters *ctr;
-    int sort_rounds;          // keys per sort thread (tile = kSortThreads x rounds)
-    int sort_first;           // first sort pass (0; 1 or 2 after shallow trees: k_fix_low)
-    uint32_t *sort_counts;    // [8][sort tiles][256]: digit counts per tile and pass
-    uint32_t *count_status;   // [count tiles]
+    int sort_first;           // digits the last tree's depth lets the sort leave out (0, 1, 2)
+    uint32_t *sort_counts;    // [8][tree-build blocks][256]: digit counts per tile and pass
     const float *size;        // n: node sizes for prevent_overlap (null: off)
     float *ssize;             // n: the same in sorted order, per iteration
 };
@@ -186,18 +165,20 @@ constexpr int kDispThreads = 512;
 
 // ---------------------------------------------------------------- kernels --
 void launch_bbox(const Buffers &b, int nblocks, cudaStream_t s);
-void launch_keys(const Buffers &b, int nsm, cudaStream_t s);
-void launch_sort(const Buffers &b, cudaStream_t s);
-void launch_fix_low(const Buffers &b, int nsm, cudaStream_t s);
-// Deepest tree levels after which the next sort may skip its two lowest
-// digits (levels 24..31) or its lowest one (levels 28..31): bodies then share
-// at most that many digits, two levels short of the skipped ones.
+// The quadtree of the current positions, one cooperative launch.
+void launch_build(const Buffers &b, bool keep_moments, int nsm, cudaStream_t s);
+size_t build_totals_bytes(int blocks);
+void build_set_smem_attr();
+// Bytes padded for vector loads of 64.
+inline size_t pad64(size_t x) { return (x + 63) & ~(size_t)63; }
+// Deepest tree levels after which the next sort may leave its two lowest
+// digits (levels 24..31) or its lowest one (levels 28..31) to the fix-up: bodies
+// then share at most that many digits, two levels short of those
+// (fa2_stats.sort_passes; the sort itself goes by the cells' sizes).
 constexpr int kShallowLevel = 22;
 constexpr int kMidLevel = 26;
 void launch_runs(const Buffers &b, int perturb, int nsm, cudaStream_t s);
-void launch_tree_count(const Buffers &b, bool keep_moments, cudaStream_t s);
 void launch_moments(const Buffers &b, cudaStream_t s);
-void launch_emit(const Buffers &b, int nsm, cudaStream_t s);
 void launch_quad_cells(const Buffers &b, int nsm, cudaStream_t s);
 void launch_traverse(const Buffers &b, const Params &p, int nblocks, cudaStream_t s);
 void launch_displace(const Buffers &b, int nsm, cudaStream_t s);
@@ -219,7 +200,6 @@ void launch_gather_xy(int n, const uint32_t *ref_of, const float2 *src_int, floa
                       cudaStream_t s);
 void launch_sorted_ref_ids(int n, const uint32_t *ref_of, const uint32_t *vals, uint32_t *out,
                            cudaStream_t s);
-void sort_set_smem_attr();
 int traverse_blocks_per_sm();
 
 }  // namespace fa2

@@ -1,13 +1,10 @@
 // fa2_kernels.cu -- the per-iteration kernels of the B200 ForceAtlas2 engine
-// around the quadtree: bounding box, Morton keys, force traversal (+ speed),
-// displacement, attraction, and the id permutations of the C ABI.  The radix
-// sort is in fa2_sort.cu, the tree build in fa2_tree.cu.
+// around the quadtree: bounding box, force traversal (+ speed), displacement,
+// attraction, and the id permutations of the C ABI.  The tree build is in
+// fa2_build.cuh.
 //
-// Keys: each body's 32 quadrant digits, computed with the reference's float
-// cell-centre arithmetic and tie rule (src/RPBHKernels.cu:217-241), form a
-// 64-bit Morton key; keys ascending give the reference's in-order body order
-// (sortd).  The tree is stored in preorder with each node's "next" index (the
-// node after its subtree), so the traversal needs no stack.
+// The tree is stored in preorder with each node's "next" index (the node
+// after its subtree), so a walk of any part of it needs no stack.
 #include <float.h>
 #include <stdint.h>
 
@@ -107,41 +104,6 @@ __global__ void __launch_bounds__(kBBoxThreads) k_bbox(int n, const float2 *__re
 // h / d >= c theta  <=>  dq - eps >= 4 c^2 d^2: no theta needed.
 __device__ __forceinline__ bool learn_keep(float dq, float wx, float wy, float eps) {
     return dq - eps >= 4.0f * kLearnMinRatio * kLearnMinRatio * (wx * wx + wy * wy);
-}
-
-// ------------------------------------------------------------------- keys --
-
-// One block per sort tile: the tile's keys, the tile's counts of the digit
-// of the first sort pass (that pass's per-tile input) and the tile's share of
-// the digit histograms of all eight passes (order-independent, so counted
-// once here).
-__global__ void __launch_bounds__(1024) k_keys(int n, int tile, int first,
-                                              const float2 *__restrict pos,
-                                              const DevState *__restrict st,
-                                              uint64_t *__restrict keys, uint32_t *__restrict vals,
-                                              IterCounters *ctr, uint32_t *__restrict counts) {
-    __shared__ unsigned s_hist[8][256];
-    if (st->err || st->poison) return;
-    for (int j = threadIdx.x; j < 8 * 256; j += blockDim.x) (&s_hist[0][0])[j] = 0;
-    __syncthreads();
-    const float rx = st->rootx, ry = st->rooty, rr = st->radius;
-    const int tile0 = blockIdx.x * tile;
-    const int tile_end = min(n, tile0 + tile);
-    for (int i = tile0 + threadIdx.x; i < tile_end; i += blockDim.x) {
-        float2 p = pos[i];
-        uint64_t key = morton_key(p.x, p.y, rx, ry, rr);
-        keys[i] = key;
-        vals[i] = (uint32_t)i;
-        // the histograms of the passes the sort runs
-        for (int ps = first; ps < 8; ++ps) atomicAdd(&s_hist[ps][(key >> (8 * ps)) & 255], 1u);
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < 8 * 256; j += blockDim.x) {
-        unsigned c = (&s_hist[0][0])[j];
-        if ((j >> 8) == first)
-            counts[((size_t)first * gridDim.x + blockIdx.x) * 256 + (j & 255)] = c;
-        if (c) atomicAdd(&(&ctr->hist[0][0])[j], c);
-    }
 }
 
 // --------------------------------------------------------------- traverse --
@@ -795,19 +757,6 @@ inline int grid_for(int n, int threads, int cap) {
 void launch_bbox(const Buffers &b, int nblocks, cudaStream_t s) {
     k_bbox<<<nblocks, kBBoxThreads, 0, s>>>(b.n, b.pos, b.bbox_partial, b.st, b.ctr);
 }
-
-void launch_keys(const Buffers &b, int nsm, cudaStream_t s) {
-    (void)nsm;
-    // the first sort pass reads buffer (first & 1), so the passes end in buffer 0
-    const int in = b.sort_first & 1;
-    k_keys<<<sort_tiles(b.n, b.sort_rounds), 1024, 0, s>>>(
-        b.n, kSortThreads * b.sort_rounds, b.sort_first, b.pos, b.st, b.keys[in], b.vals[in],
-        b.ctr, b.sort_counts);
-}
-
-
-
-
 
 namespace {
 

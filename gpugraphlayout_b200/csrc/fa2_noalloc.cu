@@ -30,11 +30,11 @@ constexpr int kMaxDevices = 64;
 constexpr size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr int tiles_of(uint32_t n, int tile) { return (int)((n + tile - 1) / tile); }
 
+constexpr int kMaxBuildBlocks = tiles_of(kMaxBodies, kBuildMinTile);
+
 // Byte offsets of the sub-buffers inside the static array, each on a
 // 256-byte boundary.  The first region is the one cleared on every call.
-constexpr size_t kZeroBytes = sizeof(IterCounters) +
-                              4 * ((size_t)8 * tiles_of(kMaxBodies, kSortTileMin) * 256 +
-                                   (size_t)tiles_of(kMaxBodies, kCountTile));
+constexpr size_t kZeroBytes = sizeof(IterCounters);
 constexpr size_t kOffZero = 0;
 constexpr size_t kOffSt = up256(kOffZero + kZeroBytes);
 constexpr size_t kOffFag = up256(kOffSt + sizeof(DevState));
@@ -45,16 +45,20 @@ constexpr size_t kOffKeys1 = up256(kOffKeys0 + 8ull * kMaxBodies);
 constexpr size_t kOffVals0 = up256(kOffKeys1 + 8ull * kMaxBodies);
 constexpr size_t kOffVals1 = up256(kOffVals0 + 4ull * kMaxBodies);
 constexpr size_t kOffLcp = up256(kOffVals1 + 4ull * kMaxBodies);
-constexpr size_t kOffGroup = up256(kOffLcp + 1ull * kMaxBodies);
+constexpr size_t kMaxRows = (kMaxBodies + 31) / 32;
+constexpr size_t kOffRowMin = up256(kOffLcp + 1ull * kMaxBodies);
+constexpr size_t kOffTileMin = up256(kOffRowMin + kMaxRows);
+constexpr size_t kOffDefer = up256(kOffTileMin + kMaxBuildBlocks);
+constexpr size_t kOffSbody = up256(kOffDefer + 4ull * (kLevels + 1) * kMaxRows);
+constexpr size_t kOffGroup = up256(kOffSbody + 16ull * kMaxBodies);
 constexpr size_t kOffBodyNode = up256(kOffGroup + 4ull * kMaxBodies);
 constexpr size_t kOffNodes = up256(kOffBodyNode + 4ull * kMaxBodies);
 constexpr size_t kOffOwner = up256(kOffNodes + 16ull * (kMaxNodes + 1));
 constexpr size_t kOffPm = up256(kOffOwner + 4ull * kMaxNodes);
 constexpr size_t kOffPxy = up256(kOffPm + 8ull * (kMaxBodies + 1));
-constexpr size_t kOffLookback =
-    up256(kOffPxy + 2ull * sizeof(__int128) * (kMaxBodies + 1));
-constexpr size_t kOffWarp =
-    up256(kOffLookback + sizeof(LookbackSums) * tiles_of(kMaxBodies, kCountTile));
+constexpr size_t kOffCounts = up256(kOffPxy + 2ull * sizeof(__int128) * (kMaxBodies + 1));
+constexpr size_t kOffTotals = up256(kOffCounts + 4ull * 8 * 256 * kMaxBuildBlocks);
+constexpr size_t kOffWarp = up256(kOffTotals + 64ull * kMaxBuildBlocks);
 constexpr size_t kOffBBox = up256(kOffWarp + 8ull * ((kMaxBodies + 31) / 32));
 constexpr size_t kScratchBytes = up256(kOffBBox + 16ull * 4 * kMaxSMs);
 static_assert(kScratchBytes < (7u << 20), "the static scratch is meant to stay near 6 MB");
@@ -108,7 +112,7 @@ int setup_device(int device, DeviceSetup *out) {
     void *p = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_scratch);
     if (e != cudaSuccess) return status_of(e);
-    sort_set_smem_attr();
+    build_set_smem_attr();
     d.trav_blocks = dp.multiProcessorCount * traverse_blocks_per_sm();
     d.base = static_cast<unsigned char *>(p);
     d.nsm = dp.multiProcessorCount;
@@ -133,7 +137,11 @@ int run(const float *d_xy, const float *d_mass, uint32_t n, const fa2_params *pr
     b.keys[1] = reinterpret_cast<uint64_t *>(base + kOffKeys1);
     b.vals[0] = reinterpret_cast<uint32_t *>(base + kOffVals0);
     b.vals[1] = reinterpret_cast<uint32_t *>(base + kOffVals1);
-    b.lcp = reinterpret_cast<int8_t *>(base + kOffLcp);
+    b.lcp = base + kOffLcp;
+    b.rowmin = base + kOffRowMin;
+    b.tilemin = base + kOffTileMin;
+    b.defer = reinterpret_cast<uint32_t *>(base + kOffDefer);
+    b.sbody = reinterpret_cast<float4 *>(base + kOffSbody);
     b.group = reinterpret_cast<uint32_t *>(base + kOffGroup);
     b.body_node = reinterpret_cast<uint32_t *>(base + kOffBodyNode);
     b.nodes = reinterpret_cast<float4 *>(base + kOffNodes);
@@ -141,16 +149,12 @@ int run(const float *d_xy, const float *d_mass, uint32_t n, const fa2_params *pr
     b.capacity = (uint32_t)kMaxNodes;
     b.pm = reinterpret_cast<long long *>(base + kOffPm);
     b.pxy = reinterpret_cast<__int128 *>(base + kOffPxy);
-    b.lookback = reinterpret_cast<LookbackSums *>(base + kOffLookback);
+    b.sort_counts = reinterpret_cast<uint32_t *>(base + kOffCounts);
+    b.build_totals = base + kOffTotals;
     b.warp_partial = reinterpret_cast<float2 *>(base + kOffWarp);
     b.bbox_partial = reinterpret_cast<float4 *>(base + kOffBBox);
     b.st = reinterpret_cast<DevState *>(base + kOffSt);
     b.ctr = reinterpret_cast<IterCounters *>(base + kOffZero);
-    b.sort_rounds = sort_rounds((int)n, d.nsm);
-    const size_t sort_counts = (size_t)8 * sort_tiles(b.n, b.sort_rounds) * 256;
-    b.sort_counts = reinterpret_cast<uint32_t *>(base + kOffZero + sizeof(IterCounters));
-    b.count_status = b.sort_counts + sort_counts;
-    const size_t zero_bytes = sizeof(IterCounters) + 4 * (sort_counts + count_tiles((int)n));
 
     Params kp{};  // every field: the kernels read all of them
     kp.k_r = prm->scale;
@@ -163,12 +167,12 @@ int run(const float *d_xy, const float *d_mass, uint32_t n, const fa2_params *pr
     kp.nsm = d.nsm;
     kp.overlap = 0;
 
-    // Must start at zero on every call: the counters, histograms, per-tile
-    // digit counts and look-back flags; the device scalars (error and
-    // coincidence flags, interaction count); the gravity + attraction term
+    // Must start at zero on every call: the counters; the device scalars
+    // (error and coincidence flags, interaction count; no last tree's cells, so
+    // the sort starts at its shortest); the gravity + attraction term
     // the traversal adds to the repulsion (zero here, so d_force receives the
     // repulsion alone).  The reference ids are the caller's indices.
-    cudaError_t e = cudaMemsetAsync(b.ctr, 0, zero_bytes, s);
+    cudaError_t e = cudaMemsetAsync(b.ctr, 0, kZeroBytes, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(b.st, 0, sizeof(DevState), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(b.fag, 0, (size_t)n * sizeof(float2), s);
     if (e != cudaSuccess) return status_of(e);
@@ -179,10 +183,7 @@ int run(const float *d_xy, const float *d_mass, uint32_t n, const fa2_params *pr
     const bool slot_was_clear = cudaPeekAtLastError() == cudaSuccess;
     k_prepare<<<(n + 255) / 256, 256, 0, s>>>(n, d_mass, const_cast<uint32_t *>(b.ref_of), b.st);
     launch_bbox(b, d.nsm * 2, s);
-    launch_keys(b, d.nsm, s);
-    launch_sort(b, s);
-    launch_tree_count(b, false, s);
-    launch_emit(b, d.nsm, s);
+    launch_build(b, false, d.nsm, s);
     launch_traverse(b, kp, d.trav_blocks, s);
     if (slot_was_clear) {
         e = cudaGetLastError();

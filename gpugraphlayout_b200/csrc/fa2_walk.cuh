@@ -1,5 +1,6 @@
 // fa2_walk.cuh -- the Barnes-Hut walk of one group of 32 sorted bodies by one
-// warp.
+// warp, shared by the single-graph traversal (fa2_kernels.cu) and the batched
+// engine (fa2_batch.cu).
 //
 // The rule is the reference's (src/RPBHKernels.cu:609-685): a cell is used as a
 // whole only if every body of the group passes d^2 + eps >= dq[level], else it
@@ -22,7 +23,7 @@
 //     lane adds the 64 terms of its own body, two per packed instruction.
 //
 // The list's order depends only on the tree and the group, so a walk's sums
-// are the same on every run, whatever block or grid it runs in.
+// are the same on every run, whatever block, grid or batch it runs in.
 //
 // Measured, k_traverse alone, one node at a time and now: 126 and 33 us on a
 // 10,000-node Barabasi-Albert graph (few groups: latency), 148 and 42 us on
@@ -213,10 +214,9 @@ __device__ __forceinline__ bool walk_accepts(const Warp &W, float cx, float cy, 
 // per round by all lanes when ON_CELLS (the learned walk's pair list).
 template <bool QUAD, bool OVERLAP, bool ON_CELLS, bool NORMAL_EPS, class OnCells>
 __device__ __forceinline__ float2 walk_group(WalkWarp<QUAD, OVERLAP> &W, const float (&dqs)[64],
-                                             const float4 *__restrict nodes,
-                                             const float2 *__restrict quad,
-                                             const uint32_t *__restrict owner,
-                                             const float *__restrict ssize, uint32_t end,
+                                             const float4 *nodes, const float2 *quad,
+                                             const uint32_t *owner, const float *ssize,
+                                             uint32_t end,
                                              float px, float py, float my_size, float eps,
                                              OnCells on_cells) {
     const int lane = threadIdx.x & 31;
@@ -244,7 +244,7 @@ __device__ __forceinline__ float2 walk_group(WalkWarp<QUAD, OVERLAP> &W, const f
             im = __ballot_sync(kFullMask, idle);
         }
         if (im == kFullMask) break;
-        const float4 r = __ldg(&nodes[idle ? 0u : node]);
+        const float4 r = nodes[idle ? 0u : node];
         const int meta = __float_as_int(r.w);
         const int lvl = meta_level(meta);
         const float thr = dqs[lvl];
@@ -259,7 +259,7 @@ __device__ __forceinline__ float2 walk_group(WalkWarp<QUAD, OVERLAP> &W, const f
             W.m[at] = r.z;
             if (QUAD) {
                 float2 q = make_float2(0.0f, 0.0f);
-                if (lvl != kBodyLevel) q = __ldg(&quad[node]);
+                if (lvl != kBodyLevel) q = quad[node];
                 W.qx[at] = q.x;
                 W.nqy[at] = -q.y;
             }

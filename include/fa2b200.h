@@ -148,7 +148,7 @@ typedef struct {
     int32_t max_level;          /* deepest cell level (root 0) */
     int32_t perturb_rounds;     /* .99 re-insertion rounds in the last step */
     int32_t device_error;       /* bit set of device-side limit hits, 0 = none:
-                                   2 tree-count wait limit, 4 more than 1024 bodies on
+                                   2 tree-build wait limit, 4 more than 1024 bodies on
                                    one 64-bit key, 8 tree larger than its buffer,
                                    16 a NaN or infinite position.  Stepping stops
                                    while one is set; fa2_set_positions clears them */
@@ -158,10 +158,14 @@ typedef struct {
     float radius, root_x, root_y;
     uint64_t interactions;      /* body-node force terms of the last traversal */
     uint64_t visits;            /* body-node acceptance tests of the last traversal */
-    int32_t sort_passes;        /* 8-bit digit passes of the last step's sorts: 8; 6
-                                   after a tree no deeper than level 22, 7 after one no
-                                   deeper than 26 (runs of keys equal in the sorted
-                                   top bits are then ordered by a fix-up pass) */
+    int32_t sort_passes;        /* 8-bit digit passes the last step's sorts take at most,
+                                   by the last tree's depth: 8; 6 after a tree no
+                                   deeper than level 22, 7 after one no deeper than 26.
+                                   The sort also leaves out low digits that the last
+                                   tree's cells hardly needed (runs of keys equal in
+                                   the sorted bits are then ordered by a fix-up, and a
+                                   run too long for it sorts again on every digit,
+                                   which counts as one of perturb_rounds) */
     uint64_t learned_pairs;     /* (group, cell) pairs the last learned iteration's walk
                                    collected for the MLP (0 without the learned
                                    correction; see fa2_set_learned_correction) */
