@@ -63,6 +63,8 @@ __global__ void __launch_bounds__(kBuildThreads, 2) k_build(BuildArgs A, int chu
         st->visits = 0;
         st->max_level = 0;  // raised in the count, after the first barrier
     }
+    // the pairs of the walk that follows (a learned iteration's)
+    if (blockIdx.x == 0 && threadIdx.x < 16) ctr->pair_count[threadIdx.x] = 0;
     GridTeam team{(int)blockIdx.x, (int)gridDim.x, &ctr->build_bar, 0u, st};
     build_tree(A, team, S, chunk);
 }

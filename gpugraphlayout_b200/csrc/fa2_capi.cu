@@ -39,6 +39,9 @@ enum Slot { S_ATTRACT, S_TRAV = 5, S_DISP, S_MOM, S_QUAD, S_LEARN, S_TREE };
 thread_local char g_last_cuda_error[192] = "";
 
 constexpr int kMaxReplayRounds = 64;
+// Iterations per captured graph of a longer step call: the gap between two
+// graphs is a few us, as long as a small graph's displacement.
+constexpr int kUnroll = 4;
 
 }  // namespace
 
@@ -66,7 +69,8 @@ struct fa2_ctx {
     cudaEvent_t evFork = nullptr, evJoin = nullptr;
     cudaEvent_t evEmitted = nullptr, evA2 = nullptr;  // the learned cells' a2 pass on stream B
     // graphs
-    cudaGraphExec_t exec = nullptr;
+    cudaGraphExec_t exec = nullptr;       // one iteration
+    cudaGraphExec_t exec_many = nullptr;  // kUnroll iterations
     cudaGraphExec_t exec_timed = nullptr;
     cudaGraph_t graph_timed = nullptr;         // kept: its nodes address exec_timed
     std::vector<cudaGraphNode_t> timed_nodes;  // event-record nodes, [slot*2 + start/end]
@@ -92,9 +96,10 @@ namespace {
 // Drops the captured iteration graphs; the next step captures them again.
 void drop_graphs(fa2_ctx *c) {
     if (c->exec) cudaGraphExecDestroy(c->exec);
+    if (c->exec_many) cudaGraphExecDestroy(c->exec_many);
     if (c->exec_timed) cudaGraphExecDestroy(c->exec_timed);
     if (c->graph_timed) cudaGraphDestroy(c->graph_timed);
-    c->exec = c->exec_timed = nullptr;
+    c->exec = c->exec_many = c->exec_timed = nullptr;
     c->graph_timed = nullptr;
 }
 
@@ -162,6 +167,7 @@ int ensure_learn_buffers(fa2_ctx *c) {
 
 void free_all(fa2_ctx *c) {
     if (c->exec) cudaGraphExecDestroy(c->exec);
+    if (c->exec_many) cudaGraphExecDestroy(c->exec_many);
     if (c->exec_timed) cudaGraphExecDestroy(c->exec_timed);
     if (c->graph_timed) cudaGraphDestroy(c->graph_timed);
     for (cudaEvent_t e : c->slot_events) cudaEventDestroy(e);
@@ -288,8 +294,9 @@ void enqueue_iteration(fa2_ctx *c, bool full, bool perturb_first, bool timed) {
     // the moment scan and per-cell second moments of the quadrupole walk
     const bool quad = c->kp.multipole >= 2;
     const bool side = full && c->overlap;  // stream B carries the attraction
-    cudaMemsetAsync(c->scratch, 0, c->scratch_bytes, A);
-    if (learn) cudaMemsetAsync(c->lb.corr, 0, ((size_t)c->n + 31) / 32 * sizeof(float2), A);
+    // A whole iteration finds its counters at zero and leaves them so; one
+    // that stopped early (the replay follows it) does not.
+    if (!full) cudaMemsetAsync(c->scratch, 0, c->scratch_bytes, A);
     if (full && !c->overlap) {
         mark(S_ATTRACT, 0, A);
         launch_attract(b, c->kp, c->plan, A);
@@ -352,10 +359,10 @@ void enqueue_iteration(fa2_ctx *c, bool full, bool perturb_first, bool timed) {
     mark(S_DISP, 1, A);
 }
 
-int capture(fa2_ctx *c, bool timed, cudaGraphExec_t *out) {
+int capture(fa2_ctx *c, bool timed, int iters, cudaGraphExec_t *out) {
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(c->sA, cudaStreamCaptureModeThreadLocal));
-    enqueue_iteration(c, true, false, timed);
+    for (int it = 0; it < iters; ++it) enqueue_iteration(c, true, false, timed);
     cudaError_t e = cudaStreamEndCapture(c->sA, &graph);
     if (e != cudaSuccess) return cuda_status(e);
     e = cudaGraphInstantiate(out, graph, cudaGraphInstantiateFlagUseNodePriority);
@@ -380,6 +387,17 @@ int capture(fa2_ctx *c, bool timed, cudaGraphExec_t *out) {
     else
         cudaGraphDestroy(graph);
     return cuda_status(e);
+}
+
+// n iterations by replaying the captured graphs (captured here when there is
+// none): kUnroll at a time, then one by one.
+int launch_iterations(fa2_ctx *c, int n) {
+    int s = FA2_OK;
+    if (n >= kUnroll && !c->exec_many && (s = capture(c, false, kUnroll, &c->exec_many))) return s;
+    if (n % kUnroll && !c->exec && (s = capture(c, false, 1, &c->exec))) return s;
+    for (; n >= kUnroll; n -= kUnroll) CK(cudaGraphLaunch(c->exec_many, c->sA));
+    for (; n > 0; --n) CK(cudaGraphLaunch(c->exec, c->sA));
+    return FA2_OK;
 }
 
 // The guard checks only an approximation other than the reference's.
@@ -465,7 +483,6 @@ void choose_sort_passes(fa2_ctx *c, const DevState &st) {
 int run_steps(fa2_ctx *c, int32_t n_iters, bool timed, std::vector<double> *kernel_sum,
               std::vector<int> *kernel_cnt) {
     if (n_iters <= 0 || c->n == 0) return FA2_OK;
-    cudaGraphExec_t *exec = timed ? &c->exec_timed : &c->exec;
     DevState st;
     int s = read_state(c, &st);
     if (s) return s;
@@ -475,10 +492,7 @@ int run_steps(fa2_ctx *c, int32_t n_iters, bool timed, std::vector<double> *kern
     while (done < n_iters) {
         choose_sort_passes(c, st);
         // (re)captured here: a guard fallback drops the graphs
-        if (!*exec) {
-            s = capture(c, timed, exec);
-            if (s) return s;
-        }
+        if (timed && !c->exec_timed && (s = capture(c, true, 1, &c->exec_timed))) return s;
         const bool guard = guard_active(c);
         const int before = st.iters_done;
         int chunk = n_iters - done;
@@ -491,13 +505,14 @@ int run_steps(fa2_ctx *c, int32_t n_iters, bool timed, std::vector<double> *kern
                 c->event_pool.push_back(e);
             }
         }
-        for (int it = 0; it < chunk; ++it) {
-            if (timed)
-                for (int q = 0; q < kNumSlots * 2; ++q)
-                    if (c->timed_nodes[q])
-                        CK(cudaGraphExecEventRecordNodeSetEvent(
-                            *exec, c->timed_nodes[q], c->event_pool[(size_t)it * kNumSlots * 2 + q]));
-            CK(cudaGraphLaunch(*exec, c->sA));
+        if (!timed && (s = launch_iterations(c, chunk))) return s;
+        for (int it = 0; timed && it < chunk; ++it) {
+            for (int q = 0; q < kNumSlots * 2; ++q)
+                if (c->timed_nodes[q])
+                    CK(cudaGraphExecEventRecordNodeSetEvent(
+                        c->exec_timed, c->timed_nodes[q],
+                        c->event_pool[(size_t)it * kNumSlots * 2 + q]));
+            CK(cudaGraphLaunch(c->exec_timed, c->sA));
         }
         s = read_state(c, &st);
         if (s) return s;
@@ -849,6 +864,7 @@ fa2_ctx *fa2_create(const fa2_graph_desc *g, const fa2_params *prm, int *status)
         cudaMemcpyAsync(b.mass, mass.data(), (size_t)n * 4, cudaMemcpyHostToDevice, A) ||
         cudaMemsetAsync(b.pos, 0, (size_t)n * 8, A) || cudaMemsetAsync(b.fprev, 0, (size_t)n * 8, A) ||
         cudaMemsetAsync(b.f, 0, (size_t)n * 8, A) || cudaMemsetAsync(b.fag, 0, (size_t)n * 8, A) ||
+        cudaMemsetAsync(c->scratch, 0, c->scratch_bytes, A) ||
         cudaMemsetAsync(b.st, 0, sizeof(DevState), A))
         return fail(FA2_ERR_CUDA);
     DevState st0;
@@ -917,7 +933,6 @@ int fa2_step_host(fa2_ctx *c, const float *xy_in, int32_t n_iters, float *xy_out
         if ((s = run_steps(c, n_iters, false, nullptr, nullptr))) return s;
         return xy_out ? fa2_get_positions(c, xy_out) : FA2_OK;
     }
-    if (n_iters > 0 && !c->exec && (s = capture(c, false, &c->exec))) return s;
     cudaStream_t A = c->sA;
     const size_t bytes = (size_t)c->n * 8;
     if (xy_in) {
@@ -933,7 +948,7 @@ int fa2_step_host(fa2_ctx *c, const float *xy_in, int32_t n_iters, float *xy_out
     CK(cudaMemcpyAsync(c->h_before, &c->b.st->iters_done, 2 * sizeof(int),
                        cudaMemcpyDeviceToHost, A));
     c->last_perturb_rounds = 0;
-    for (int it = 0; it < n_iters; ++it) CK(cudaGraphLaunch(c->exec, A));
+    if ((s = launch_iterations(c, n_iters))) return s;
     CK(cudaMemcpyAsync(c->h_state, c->b.st, sizeof(DevState), cudaMemcpyDeviceToHost, A));
     if (xy_out) {
         launch_gather_xy((int)c->n, c->b.ref_of, c->b.pos, c->stage_xy, A);
@@ -1434,6 +1449,8 @@ int fa2_learn_collect(fa2_learn_set *set, fa2_ctx *c, float theta, int32_t multi
     launch_traverse_learn(b, kp, c->lb, c->trav_blocks, A);
     launch_learn_targets(b, kp, c->lb, set->st_feat, set->st_tgt, set->st_w, set->st_key,
                          set->st_count, (uint64_t)set->st_cap, c->nsm, A);
+    // the walk's counters, which no displacement follows here to clear
+    CK(cudaMemsetAsync(&b.ctr->trav_ticket, 0, 2 * sizeof(unsigned), A));
     CK(cudaGetLastError());
     DevState st;
     s = read_state(c, &st);

@@ -64,6 +64,7 @@ __device__ void bbox_finish(float4 a, bool bad, float4 *__restrict partial, unsi
     }
     __syncthreads();
     if (!s_last) return;
+    if (threadIdx.x == 0) *done = 0;  // for the next launch
     __threadfence();
     a = make_float4(FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX);
     for (int b = threadIdx.x; b < (int)gridDim.x; b += THREADS) a = bbox_merge(a, __ldcg(&partial[b]));
@@ -144,7 +145,10 @@ __global__ void __launch_bounds__(kTravThreads, kTravWarpsPerSm *kWarp / kTravTh
     if (st->err || st->poison) return;
     if (threadIdx.x == 0) {
         walk_thresholds(st->radius, prm, s_dq);
-        if (blockIdx.x == 0) st->trav_radius = st->radius;
+        if (blockIdx.x == 0) {
+            st->trav_radius = st->radius;
+            ctr->build_bar = 0;  // the build is done; for the next one
+        }
     }
     __syncthreads();
     const uint32_t end = st->tree_nodes;
@@ -184,6 +188,7 @@ __global__ void __launch_bounds__(kTravThreads, kTravWarpsPerSm *kWarp / kTravTh
                 t2 += __shfl_xor_sync(kFull, t2, o);
             }
             if (lane == 0) {
+                lb.corr[w] = make_float2(0.0f, 0.0f);  // the MLP adds to it
                 lb.ggeo[2 * w] = make_float4(gx, gy, t0 / cnt, cnt);
                 lb.ggeo[2 * w + 1] = make_float4(t1 / cnt, t2 / cnt, 0.0f, 0.0f);
             }
@@ -498,7 +503,11 @@ __global__ void __launch_bounds__(kDispThreads, 2048 / kDispThreads) k_displace(
         bad |= !(isfinite(p.x) && isfinite(p.y));
     }
     bbox_finish<kDispThreads>(a, bad, partial, &ctr->disp_done, st);
-    if (blockIdx.x == 0 && threadIdx.x == 0) st->iters_done += 1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->iters_done += 1;
+        ctr->trav_ticket = 0;  // the traversal is done; for the next one
+        ctr->trav_done = 0;
+    }
 }
 
 // ---------------------------------------------------------------- attract --

@@ -231,9 +231,14 @@ __global__ void __launch_bounds__(kQuadThreads, 4) k_quad_cells(const float4 *__
                                                              const long long *__restrict pm,
                                                              const Moments *__restrict pmom,
                                                              float2 *__restrict quad,
-                                                             DevState *st) {
+                                                             uint32_t *mom_status, int mom_tiles,
+                                                             IterCounters *ctr, DevState *st) {
     __shared__ uint32_t s_q[kQuadThreads / kWarp][64];
     if (st->err || st->poison) return;
+    // the moment scan is done: its ticket and flags for the next one
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctr->mom_ticket = 0;
+    for (int t = blockIdx.x * kQuadThreads + threadIdx.x; t < mom_tiles; t += gridDim.x * kQuadThreads)
+        mom_status[t] = 0;
     const uint32_t total = st->tree_nodes;
     const float radius = st->radius;
     const int lane = threadIdx.x & 31;
@@ -280,7 +285,7 @@ void launch_runs(const Buffers &b, int perturb, int nsm, cudaStream_t s) {
 
 void launch_quad_cells(const Buffers &b, int nsm, cudaStream_t s) {
     k_quad_cells<<<grid_for(b.n, kQuadThreads, nsm * 4), kQuadThreads, 0, s>>>(
-        b.nodes, b.owner, b.pm, b.pmom, b.quad, b.st);
+        b.nodes, b.owner, b.pm, b.pmom, b.quad, b.mom_status, mom_tiles(b.n), b.ctr, b.st);
 }
 
 }  // namespace fa2
