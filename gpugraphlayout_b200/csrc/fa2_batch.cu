@@ -700,6 +700,11 @@ __global__ void __launch_bounds__(T, kBatchThreadsPerSm / T) k_batch(BatchArgs A
     }
 }
 
+__global__ void k_clear_errors(int n, BatchSpeed *__restrict speed) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < n) speed[g].err = 0;
+}
+
 size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 SlotLayout make_layout(uint32_t nmax) {
@@ -1128,13 +1133,9 @@ int fa2_batch_set_positions(fa2_batch *b, const float *xy) {
     if (!b->total_nodes) return FA2_OK;
     BCK(cudaMemcpyAsync(b->args.pos, xy, b->total_nodes * 8, cudaMemcpyHostToDevice, b->stream));
     // new positions clear the graphs' device errors, which depend on them
-    std::vector<BatchSpeed> sp(b->num_graphs);
-    BCK(cudaMemcpyAsync(sp.data(), b->args.speed, sp.size() * sizeof(BatchSpeed),
-                        cudaMemcpyDeviceToHost, b->stream));
-    BCK(cudaStreamSynchronize(b->stream));
-    for (BatchSpeed &x : sp) x.err = 0;
-    BCK(cudaMemcpyAsync(b->args.speed, sp.data(), sp.size() * sizeof(BatchSpeed),
-                        cudaMemcpyHostToDevice, b->stream));
+    k_clear_errors<<<(b->num_graphs + 255) / 256, 256, 0, b->stream>>>((int)b->num_graphs,
+                                                                       b->args.speed);
+    BCK(cudaGetLastError());
     BCK(cudaStreamSynchronize(b->stream));
     return FA2_OK;
 }

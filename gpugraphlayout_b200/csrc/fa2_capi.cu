@@ -62,7 +62,11 @@ struct fa2_ctx {
     size_t scratch_bytes = 0;
     float2 *stage_xy = nullptr;    // n, reference order
     DevState *h_state = nullptr;   // pinned: the state after fa2_step_host's iterations
-    int *h_before = nullptr;       // pinned: iters_done and resorts before them
+    // what the host knows of the device's state without asking: the last state
+    // it read, if nothing has run since; whether the counters are at zero;
+    // whether an error bit may be set
+    DevState seen{};
+    bool seen_ok = false, counters_zero = false, maybe_err = true;
     uint32_t *stage_ids = nullptr; // n
     int bbox_blocks = 0, trav_blocks = 0;
     cudaStream_t sA = nullptr, sB = nullptr;
@@ -181,7 +185,6 @@ void free_all(fa2_ctx *c) {
     if (c->sA) cudaStreamDestroy(c->sA);
     if (c->sB) cudaStreamDestroy(c->sB);
     if (c->h_state) cudaFreeHost(c->h_state);
-    if (c->h_before) cudaFreeHost(c->h_before);
 }
 
 // Nodes in degree-descending order (ties by reference id), a symmetric CSR
@@ -294,8 +297,8 @@ void enqueue_iteration(fa2_ctx *c, bool full, bool perturb_first, bool timed) {
     // the moment scan and per-cell second moments of the quadrupole walk
     const bool quad = c->kp.multipole >= 2;
     const bool side = full && c->overlap;  // stream B carries the attraction
-    // A whole iteration finds its counters at zero and leaves them so; one
-    // that stopped early (the replay follows it) does not.
+    // A whole iteration finds its counters at zero (clear_counters) and leaves
+    // them so; one that stopped early, which this replays, does not.
     if (!full) cudaMemsetAsync(c->scratch, 0, c->scratch_bytes, A);
     if (full && !c->overlap) {
         mark(S_ATTRACT, 0, A);
@@ -389,10 +392,52 @@ int capture(fa2_ctx *c, bool timed, int iters, cudaGraphExec_t *out) {
     return cuda_status(e);
 }
 
+// The state as the device has it now, every launch done.
+void note_state(fa2_ctx *c, const DevState &st) {
+    c->seen = st;
+    c->seen_ok = true;
+    c->maybe_err = st.err != 0;
+}
+
+int read_state(fa2_ctx *c, DevState *st) {
+    c->seen_ok = false;
+    CK(cudaMemcpyAsync(st, c->b.st, sizeof(DevState), cudaMemcpyDeviceToHost, c->sA));
+    CK(cudaStreamSynchronize(c->sA));
+    note_state(c, *st);
+    return FA2_OK;
+}
+
+// Before anything that counts: the counters at zero.  A whole iteration leaves
+// them so; c->counters_zero is set again once the state shows that the last
+// one was.
+int clear_counters(fa2_ctx *c) {
+    if (!c->counters_zero) CK(cudaMemsetAsync(c->scratch, 0, c->scratch_bytes, c->sA));
+    c->counters_zero = false;
+    return FA2_OK;
+}
+
+// New positions in c->stage_xy, reference order: the nodes' positions and the
+// root cell of the next tree.  Device errors of earlier positions are cleared
+// (the pass flags non-finite ones).
+int place_positions(fa2_ctx *c) {
+    if (c->maybe_err) CK(cudaMemsetAsync(&c->b.st->err, 0, sizeof(int), c->sA));
+    c->maybe_err = true;
+    c->seen_ok = false;
+    const bool zero = c->counters_zero;
+    int s = clear_counters(c);
+    if (s) return s;
+    launch_place(c->b, c->stage_xy, c->bbox_blocks, c->sA);
+    c->counters_zero = zero;  // the pass clears its own
+    return FA2_OK;
+}
+
 // n iterations by replaying the captured graphs (captured here when there is
 // none): kUnroll at a time, then one by one.
 int launch_iterations(fa2_ctx *c, int n) {
-    int s = FA2_OK;
+    if (n <= 0) return FA2_OK;
+    int s = clear_counters(c);
+    if (s) return s;
+    c->seen_ok = false;
     if (n >= kUnroll && !c->exec_many && (s = capture(c, false, kUnroll, &c->exec_many))) return s;
     if (n % kUnroll && !c->exec && (s = capture(c, false, 1, &c->exec))) return s;
     for (; n >= kUnroll; n -= kUnroll) CK(cudaGraphLaunch(c->exec_many, c->sA));
@@ -448,12 +493,6 @@ int guard_check(fa2_ctx *c) {
     return FA2_OK;
 }
 
-int read_state(fa2_ctx *c, DevState *st) {
-    CK(cudaMemcpyAsync(st, c->b.st, sizeof(DevState), cudaMemcpyDeviceToHost, c->sA));
-    CK(cudaStreamSynchronize(c->sA));
-    return FA2_OK;
-}
-
 // Replays a poisoned iteration until no coincident bodies remain.
 int resolve_poison(fa2_ctx *c, DevState *st) {
     int rounds = 0;
@@ -483,8 +522,8 @@ void choose_sort_passes(fa2_ctx *c, const DevState &st) {
 int run_steps(fa2_ctx *c, int32_t n_iters, bool timed, std::vector<double> *kernel_sum,
               std::vector<int> *kernel_cnt) {
     if (n_iters <= 0 || c->n == 0) return FA2_OK;
-    DevState st;
-    int s = read_state(c, &st);
+    DevState st = c->seen;
+    int s = c->seen_ok ? FA2_OK : read_state(c, &st);
     if (s) return s;
     int done = 0;
     c->last_perturb_rounds = 0;
@@ -506,6 +545,7 @@ int run_steps(fa2_ctx *c, int32_t n_iters, bool timed, std::vector<double> *kern
             }
         }
         if (!timed && (s = launch_iterations(c, chunk))) return s;
+        if (timed && (s = clear_counters(c))) return s;
         for (int it = 0; timed && it < chunk; ++it) {
             for (int q = 0; q < kNumSlots * 2; ++q)
                 if (c->timed_nodes[q])
@@ -538,6 +578,7 @@ int run_steps(fa2_ctx *c, int32_t n_iters, bool timed, std::vector<double> *kern
             done += 1;  // the replayed iteration completed
             completed += 1;
         }
+        c->counters_zero = true;  // the last iteration was a whole one
         if (guard) {
             c->guard_left -= completed;
             if (c->guard_left <= 0) {
@@ -847,8 +888,7 @@ fa2_ctx *fa2_create(const fa2_graph_desc *g, const fa2_params *prm, int *status)
         cudaEventCreateWithFlags(&c->evJoin, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->evEmitted, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->evA2, cudaEventDisableTiming) != cudaSuccess ||
-        cudaMallocHost(&c->h_state, sizeof(DevState)) != cudaSuccess ||
-        cudaMallocHost(&c->h_before, 2 * sizeof(int)) != cudaSuccess)
+        cudaMallocHost(&c->h_state, sizeof(DevState)) != cudaSuccess)
         return fail(FA2_ERR_CUDA);
     c->slot_events.resize(kNumSlots * 2);
     for (auto &e : c->slot_events)
@@ -895,12 +935,8 @@ int fa2_set_positions(fa2_ctx *c, const float *xy) {
     if (c->n == 0) return FA2_OK;
     const size_t bytes = (size_t)c->n * 8;
     CK(cudaMemcpyAsync(c->stage_xy, xy, bytes, cudaMemcpyHostToDevice, c->sA));
-    launch_scatter_xy((int)c->n, c->b.ref_of, c->stage_xy, c->b.pos, c->sA);
-    // the root cell of the next tree comes from these positions; device
-    // errors of earlier positions are cleared (k_bbox flags non-finite ones)
-    CK(cudaMemsetAsync(c->scratch, 0, c->scratch_bytes, c->sA));
-    CK(cudaMemsetAsync(&c->b.st->err, 0, sizeof(int), c->sA));
-    launch_bbox(c->b, c->bbox_blocks, c->sA);
+    int s = place_positions(c);
+    if (s) return s;
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->sA));
     return FA2_OK;
@@ -910,7 +946,7 @@ int fa2_get_positions(fa2_ctx *c, float *xy) {
     if (!c || (!xy && c->n)) return FA2_ERR_INVALID_ARGUMENT;
     CK(cudaSetDevice(c->device));
     if (c->n == 0) return FA2_OK;
-    launch_gather_xy((int)c->n, c->b.ref_of, c->b.pos, c->stage_xy, c->sA);
+    launch_gather_xy((int)c->n, c->b.ref_of, c->b.pos, c->stage_xy, nullptr, nullptr, c->sA);
     CK(cudaMemcpyAsync(xy, c->stage_xy, (size_t)c->n * 8, cudaMemcpyDeviceToHost, c->sA));
     CK(cudaStreamSynchronize(c->sA));
     return FA2_OK;
@@ -935,32 +971,32 @@ int fa2_step_host(fa2_ctx *c, const float *xy_in, int32_t n_iters, float *xy_out
     }
     cudaStream_t A = c->sA;
     const size_t bytes = (size_t)c->n * 8;
+    const bool known = c->seen_ok;  // iterations and sorts done so far
     if (xy_in) {
         // fa2_set_positions without its synchronisation
         CK(cudaMemcpyAsync(c->stage_xy, xy_in, bytes, cudaMemcpyHostToDevice, A));
-        launch_scatter_xy((int)c->n, c->b.ref_of, c->stage_xy, c->b.pos, A);
-        CK(cudaMemsetAsync(c->scratch, 0, c->scratch_bytes, A));
-        CK(cudaMemsetAsync(&c->b.st->err, 0, sizeof(int), A));
-        launch_bbox(c->b, c->bbox_blocks, A);
+        if ((s = place_positions(c))) return s;
     }
-    static_assert(offsetof(DevState, resorts) == offsetof(DevState, iters_done) + sizeof(int),
-                  "iters_done and resorts are read with one copy");
-    CK(cudaMemcpyAsync(c->h_before, &c->b.st->iters_done, 2 * sizeof(int),
-                       cudaMemcpyDeviceToHost, A));
+    DevState st = c->seen;
+    if (!known && (s = read_state(c, &st))) return s;
+    const int before = st.iters_done;
+    c->resorts_before = st.resorts;
     c->last_perturb_rounds = 0;
     if ((s = launch_iterations(c, n_iters))) return s;
-    CK(cudaMemcpyAsync(c->h_state, c->b.st, sizeof(DevState), cudaMemcpyDeviceToHost, A));
     if (xy_out) {
-        launch_gather_xy((int)c->n, c->b.ref_of, c->b.pos, c->stage_xy, A);
+        launch_gather_xy((int)c->n, c->b.ref_of, c->b.pos, c->stage_xy, c->b.st, c->h_state, A);
         CK(cudaMemcpyAsync(xy_out, c->stage_xy, bytes, cudaMemcpyDeviceToHost, A));
+    } else {
+        CK(cudaMemcpyAsync(c->h_state, c->b.st, sizeof(DevState), cudaMemcpyDeviceToHost, A));
     }
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(A));
-    DevState st = *c->h_state;
-    c->resorts_before = c->h_before[1];
+    st = *c->h_state;
+    note_state(c, st);
     if (st.err) return FA2_ERR_DEVICE_LIMIT;
-    int completed = st.iters_done - c->h_before[0];
+    int completed = st.iters_done - before;
     if (completed == n_iters && !st.poison) {
+        c->counters_zero = true;
         choose_sort_passes(c, st);
         return FA2_OK;
     }
@@ -1051,7 +1087,7 @@ int fa2_get_forces(fa2_ctx *c, float *f_total, float *f_attr_grav) {
     float2 *srcs[2] = {c->b.f, c->b.fag};
     for (int q = 0; q < 2; ++q) {
         if (!outs[q]) continue;
-        launch_gather_xy((int)c->n, c->b.ref_of, srcs[q], c->stage_xy, c->sA);
+        launch_gather_xy((int)c->n, c->b.ref_of, srcs[q], c->stage_xy, nullptr, nullptr, c->sA);
         CK(cudaMemcpyAsync(outs[q], c->stage_xy, (size_t)c->n * 8, cudaMemcpyDeviceToHost, c->sA));
         CK(cudaStreamSynchronize(c->sA));
     }
@@ -1100,7 +1136,7 @@ int fa2_get_speed_state(fa2_ctx *c, float *global_speed, float *speed_efficiency
     if (global_speed) *global_speed = st.global_speed;
     if (speed_efficiency) *speed_efficiency = st.speed_efficiency;
     if (f_prev && c->n) {
-        launch_gather_xy((int)c->n, c->b.ref_of, c->b.fprev, c->stage_xy, c->sA);
+        launch_gather_xy((int)c->n, c->b.ref_of, c->b.fprev, c->stage_xy, nullptr, nullptr, c->sA);
         CK(cudaMemcpyAsync(f_prev, c->stage_xy, (size_t)c->n * 8, cudaMemcpyDeviceToHost, c->sA));
         CK(cudaStreamSynchronize(c->sA));
     }
@@ -1440,7 +1476,10 @@ int fa2_learn_collect(fa2_learn_set *set, fa2_ctx *c, float theta, int32_t multi
     kp.multipole = multipole;
     Buffers b = c->b;
     cudaStream_t A = c->sA;
-    CK(cudaMemsetAsync(c->scratch, 0, c->scratch_bytes, A));
+    // no displacement follows this walk to clear its counters
+    c->counters_zero = false;
+    if ((s = clear_counters(c))) return s;
+    c->seen_ok = false;
     CK(cudaMemsetAsync(set->st_count, 0, sizeof(unsigned long long), A));
     launch_build(b, multipole >= 2, c->nsm, A);
     if (multipole >= 2) launch_moments(b, A);
@@ -1449,8 +1488,6 @@ int fa2_learn_collect(fa2_learn_set *set, fa2_ctx *c, float theta, int32_t multi
     launch_traverse_learn(b, kp, c->lb, c->trav_blocks, A);
     launch_learn_targets(b, kp, c->lb, set->st_feat, set->st_tgt, set->st_w, set->st_key,
                          set->st_count, (uint64_t)set->st_cap, c->nsm, A);
-    // the walk's counters, which no displacement follows here to clear
-    CK(cudaMemsetAsync(&b.ctr->trav_ticket, 0, 2 * sizeof(unsigned), A));
     CK(cudaGetLastError());
     DevState st;
     s = read_state(c, &st);

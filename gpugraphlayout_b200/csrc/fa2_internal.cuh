@@ -39,7 +39,7 @@ struct DevState {
     int poison;          // coincident bodies seen: this iteration is replayed
     int err;             // kErr* bits
     int iters_done;      // completed iterations
-    int resorts;         // sorts done again on every digit (read with iters_done)
+    int resorts;         // sorts done again on every digit
     uint32_t tree_nodes; // nodes of the last quadtree
     int max_level;
     float swg_sum, etra_sum;
@@ -196,8 +196,11 @@ void launch_attract(const Buffers &b, const Params &p, const AttractPlan &plan, 
 void launch_sorted_sizes(const Buffers &b, cudaStream_t s);
 void launch_scatter_xy(int n, const uint32_t *ref_of, const float2 *src_ref, float2 *dst_int,
                        cudaStream_t s);
+// Positions from reference order, and in reference order; with host_st, the
+// device state to that pinned host copy as well.
+void launch_place(const Buffers &b, const float2 *src_ref, int nblocks, cudaStream_t s);
 void launch_gather_xy(int n, const uint32_t *ref_of, const float2 *src_int, float2 *dst_ref,
-                      cudaStream_t s);
+                      const DevState *st, DevState *host_st, cudaStream_t s);
 void launch_sorted_ref_ids(int n, const uint32_t *ref_of, const uint32_t *vals, uint32_t *out,
                            cudaStream_t s);
 int traverse_blocks_per_sm();

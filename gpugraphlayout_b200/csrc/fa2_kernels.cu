@@ -84,15 +84,20 @@ __device__ void bbox_finish(float4 a, bool bad, float4 *__restrict partial, unsi
     }
 }
 
-// Bounding box of the current positions (run after positions are set from
-// the host; during stepping the displacement pass computes it).
-__global__ void __launch_bounds__(kBBoxThreads) k_bbox(int n, const float2 *__restrict pos,
+// Bounding box of the current positions (during stepping the displacement pass
+// computes it).  With a source, the positions are first taken from there, in
+// reference order (positions set from the host).
+template <bool PLACE>
+__global__ void __launch_bounds__(kBBoxThreads) k_bbox(int n, float2 *__restrict pos,
+                                                       const float2 *__restrict src_ref,
+                                                       const uint32_t *__restrict ref_of,
                                                        float4 *__restrict partial,
                                                        DevState *st, IterCounters *ctr) {
     float4 a = make_float4(FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX);
     bool bad = false;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float2 p = pos[i];
+        const float2 p = PLACE ? src_ref[ref_of[i]] : pos[i];
+        if (PLACE) pos[i] = p;
         a = bbox_merge(a, make_float4(p.x, p.x, p.y, p.y));
         bad |= !(isfinite(p.x) && isfinite(p.y));
     }
@@ -743,9 +748,16 @@ __global__ void k_scatter_xy(int n, const uint32_t *__restrict ref_of,
 }
 
 __global__ void k_gather_xy(int n, const uint32_t *__restrict ref_of,
-                            const float2 *__restrict src_int, float2 *__restrict dst_ref) {
+                            const float2 *__restrict src_int, float2 *__restrict dst_ref,
+                            const DevState *__restrict st, DevState *__restrict host_st) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         dst_ref[ref_of[i]] = src_int[i];
+    // the state beside them, straight into the caller's pinned copy
+    constexpr int kWords = (int)(sizeof(DevState) / sizeof(uint32_t));
+    if (host_st && blockIdx.x == 0)
+        for (int j = threadIdx.x; j < kWords; j += blockDim.x)
+            reinterpret_cast<volatile uint32_t *>(host_st)[j] =
+                reinterpret_cast<const uint32_t *>(st)[j];
 }
 
 __global__ void k_sorted_ref_ids(int n, const uint32_t *__restrict ref_of,
@@ -764,7 +776,13 @@ inline int grid_for(int n, int threads, int cap) {
 // ---------------------------------------------------------------- launchers --
 
 void launch_bbox(const Buffers &b, int nblocks, cudaStream_t s) {
-    k_bbox<<<nblocks, kBBoxThreads, 0, s>>>(b.n, b.pos, b.bbox_partial, b.st, b.ctr);
+    k_bbox<false><<<nblocks, kBBoxThreads, 0, s>>>(b.n, b.pos, nullptr, nullptr, b.bbox_partial,
+                                                   b.st, b.ctr);
+}
+
+void launch_place(const Buffers &b, const float2 *src_ref, int nblocks, cudaStream_t s) {
+    k_bbox<true><<<nblocks, kBBoxThreads, 0, s>>>(b.n, b.pos, src_ref, b.ref_of, b.bbox_partial,
+                                                  b.st, b.ctr);
 }
 
 namespace {
@@ -869,8 +887,8 @@ void launch_scatter_xy(int n, const uint32_t *ref_of, const float2 *src_ref, flo
 }
 
 void launch_gather_xy(int n, const uint32_t *ref_of, const float2 *src_int, float2 *dst_ref,
-                      cudaStream_t s) {
-    k_gather_xy<<<grid_for(n, 256, 4096), 256, 0, s>>>(n, ref_of, src_int, dst_ref);
+                      const DevState *st, DevState *host_st, cudaStream_t s) {
+    k_gather_xy<<<grid_for(n, 256, 4096), 256, 0, s>>>(n, ref_of, src_int, dst_ref, st, host_st);
 }
 
 void launch_sorted_ref_ids(int n, const uint32_t *ref_of, const uint32_t *vals, uint32_t *out,
