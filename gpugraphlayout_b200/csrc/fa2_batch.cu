@@ -1,15 +1,18 @@
 // fa2_batch.cu -- many independent graphs laid out in one persistent launch.
 //
 // Each graph is small next to the GPU (tens to tens of thousands of nodes),
-// so one CTA runs the whole ForceAtlas2 iteration of one graph: gravity and
-// attraction, bounding box, Morton keys, a block-level radix sort, the tree
-// (counts, prefix sums, nodes), the warp-vote traversal, the speed rule and
-// the displacement -- the same arithmetic as the single-graph kernels, with
-// every reduction and scan inside the block.  No CTA waits on another.  The
-// CTAs of a grid that fills the GPU take graphs from a queue, largest first,
+// so one team, a block or a cluster of up to eight, runs the whole ForceAtlas2
+// iteration of one graph: gravity and attraction, bounding box, the tree
+// (build_tree), the walk (walk_group), the speed rule and the displacement --
+// the same code and arithmetic as the single-graph kernels.  Only the blocks
+// of a cluster wait on one another, at the cluster's hardware barrier.  The
+// teams of a grid that fills the GPU take graphs from a queue, largest first,
 // and run `iters` iterations of a graph before taking the next, so a graph's
-// working set stays in L2 across its iterations.  Per-CTA scratch lives in
-// one slot per CTA, sized for the largest graph of the batch.
+// working set stays in L2 across its iterations.  A team's scratch is one
+// slot, sized for the largest graph of its class.
+//
+// Why clusters: with one block per graph the batch took as long as its
+// largest graph, 1.7 ms for 20,000 nodes, while the other SMs ran dry.
 //
 // The reference has no batched mode: it lays out one graph per process, with
 // its speed and tree state in device statics (src/RPFA2Kernels.cu:29-33,
@@ -23,6 +26,7 @@
 #include <vector>
 
 #include "../../include/fa2b200.h"
+#include "fa2_build.cuh"
 #include "fa2_device.cuh"
 #include "fa2_walk.cuh"
 
@@ -30,13 +34,9 @@ namespace fa2 {
 
 namespace {
 
-// Threads per CTA (T) is a template parameter: 256, 512 or 1024.  Every
-// result is the same for each (stable sort, exact integer sums, per-warp
-// walks, fixed-order speed sums); only the speed differs.
-constexpr int kBRounds = 4;                       // keys per thread in a sort chunk
-// A sort that skips low digits leaves runs of keys equal in the digits it
-// sorted; a run longer than this sends the graph back to a sort on every digit.
-constexpr int kBMaxRun = 128;
+// Every result is the same for each team (stable sort, exact integer sums,
+// per-warp walks, fixed-order speed sums); only the speed differs.
+constexpr int kMaxTeam = 8;                       // blocks per graph (a portable cluster)
 constexpr uint32_t kBatchMaxNodes = FA2_BATCH_MAX_NODES;  // nodes per graph
 constexpr int kErrPoisonRounds = 1 << 9;          // coincident bodies kept reappearing
 
@@ -51,9 +51,22 @@ struct BatchSpeed {
     int perturb_rounds;  // .99 re-insertion rounds of its last iteration
 };
 
-// Offsets of one CTA's scratch slot, in bytes, each 256-byte aligned.
+// Control block of one team's slot, in global memory: what its blocks share.
+struct BatchCtl {
+    int graph;     // index in the queue order
+    int ticket;    // groups handed out in the walk
+    int err, poison, resort, resorts, deep;
+    int cells[kCellLevels];
+    uint32_t tree_nodes;
+    int max_level;
+    int bad;       // a block saw a NaN or infinite position
+    float4 box[kMaxTeam];  // the blocks' boxes: min x, max x, min y, max y
+};
+
+// Offsets of one team's scratch slot, in bytes, each 256-byte aligned.
 struct SlotLayout {
-    size_t keys0, keys1, vals0, vals1, lcp, group, body_node, owner, nodes, pm, pxy, fa, f, gpart;
+    size_t ctl, keys0, keys1, vals0, vals1, sbody, lcp, rowmin, tilemin, defer, group, body_node,
+        owner, nodes, pm, pxy, counts, totals, fa, f, gpart;
     size_t bytes;
     uint32_t cap;  // tree nodes a slot holds
 };
@@ -74,108 +87,56 @@ struct BatchArgs {
     Params prm;
     float jitter_tolerance, k_s_max;
     int iters;
+    int chunk;                  // keys the sort stages in shared memory
 };
 
-struct NodeSums {
-    uint32_t g;
-    long long m;
-    i128 x, y;
+// The blocks of one cluster, or one block alone.
+struct ClusterTeam {
+    int rank, size;
+    __device__ __forceinline__ bool sync() {
+        if (size == 1)
+            __syncthreads();
+        else
+            asm volatile(
+                "barrier.cluster.arrive.release;\n\t"
+                "barrier.cluster.wait.acquire;" ::
+                    : "memory");
+        return true;
+    }
 };
 
-__device__ __forceinline__ void sums_add(NodeSums &a, const NodeSums &b) {
-    a.g += b.g;
-    a.m += b.m;
-    a.x += b.x;
-    a.y += b.y;
-}
-
-__device__ __forceinline__ NodeSums shfl_up_sums(const NodeSums &v, int o) {
-    NodeSums t;
-    t.g = __shfl_up_sync(kFullMask, v.g, o);
-    t.m = __shfl_up_sync(kFullMask, v.m, o);
-    t.x = shfl_up_i128(v.x, o);
-    t.y = shfl_up_i128(v.y, o);
-    return t;
-}
-
-// Shared memory of the batch kernel (dynamic: over 48 KB with 1024 threads).
-// The sort's histograms and the warps' walks take turns.
+// Shared memory of the batch kernel (dynamic).  The build and the warps' walks
+// take turns.
 template <int T>
-struct BatchSmem {
-    union {
-        uint32_t whist[T / kWarp][256];
-        WalkWarp<false, false> walk[T / kWarp];
-    };
-    uint32_t qsum[4][256];
-    uint32_t base[256];
-    uint32_t coff[256];
-    NodeSums wsum[T / kWarp];
-    NodeSums carry;
-    float4 wbox[T / kWarp];
+struct BatchShared {
     float dq[64];
-    float2 wred[T / kWarp];
+    float4 wbox[T / kWarp];
     float rx, ry, radius;
-    uint32_t total_nodes;
-    int ticket;
-    int graph;
-    int err, poison;
-    int maxlev;   // deepest cell level of the last tree (phase_count)
-    int resort;   // a run of the partial sort was too long: sort on every digit
     float gs, se;
 };
-
-// Block-wide exclusive scan of NodeSums; *total receives the block's sum.
-// Every thread of the block calls it.
 template <int T>
-__device__ NodeSums block_scan(NodeSums v, BatchSmem<T> &S, NodeSums *total) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    NodeSums inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const NodeSums t = shfl_up_sums(inc, o);
-        if (lane >= o) sums_add(inc, t);
-    }
-    if (lane == 31) S.wsum[wid] = inc;
-    __syncthreads();
-    if (wid == 0) {
-        NodeSums w = lane < T / kWarp ? S.wsum[lane] : NodeSums{0, 0, 0, 0}, wi = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const NodeSums t = shfl_up_sums(wi, o);
-            if (lane >= o) sums_add(wi, t);
-        }
-        NodeSums ex = wi;  // exclusive = inclusive - own
-        ex.g -= w.g;
-        ex.m -= w.m;
-        ex.x -= w.x;
-        ex.y -= w.y;
-        if (lane < T / kWarp) S.wsum[lane] = ex;
-        if (lane == 31) S.carry = wi;  // block total, read below before reuse
-    }
-    __syncthreads();
-    NodeSums out = S.wsum[wid];
-    out.g += inc.g - v.g;
-    out.m += inc.m - v.m;
-    out.x += inc.x - v.x;
-    out.y += inc.y - v.y;
-    *total = S.carry;
-    __syncthreads();
-    return out;
+constexpr size_t kBatchHead = (sizeof(BatchShared<T>) + 63) & ~(size_t)63;
+template <int T>
+size_t batch_smem_bytes(int chunk) {
+    return kBatchHead<T> + std::max(build_smem_bytes<T>(chunk),
+                                            sizeof(WalkWarp<false, false>) * (T / kWarp));
 }
 
-template <typename T>
-__device__ __forceinline__ T *slot_ptr(char *slot, size_t off) {
-    return reinterpret_cast<T *>(slot + off);
+template <typename U>
+__device__ __forceinline__ U *slot_ptr(char *slot, size_t off) {
+    return reinterpret_cast<U *>(slot + off);
 }
 
 // --------------------------------------------------------------- phases --
 
 // Gravity + attraction of the graph's nodes (8 lanes per row), into fa.
 template <int T, bool LINLOG>
-__device__ void phase_attract(const BatchArgs &A, uint32_t base, uint32_t n, float2 *fa) {
+__device__ void phase_attract(const BatchArgs &A, const ClusterTeam &team, uint32_t base,
+                              uint32_t n, float2 *fa) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int sub = lane >> 3, l8 = lane & 7;
-    for (uint32_t r0 = (uint32_t)wid * 4; r0 < n; r0 += (T / kWarp) * 4) {
+    const uint32_t warp = (uint32_t)(team.rank * (T / kWarp) + wid);
+    for (uint32_t r0 = warp * 4; r0 < n; r0 += (uint32_t)team.size * (T / kWarp) * 4) {
         const uint32_t row = r0 + (uint32_t)sub;
         const bool valid = row < n;
         float ax = 0.0f, ay = 0.0f;
@@ -212,19 +173,19 @@ __device__ void phase_attract(const BatchArgs &A, uint32_t base, uint32_t n, flo
 }
 
 // Bounding box and root cell of the graph (BoundingBoxKernel,
-// src/RPBHKernels.cu:70-157), into S.rx, S.ry, S.radius.
+// src/RPBHKernels.cu:70-157), into S.rx, S.ry, S.radius of every block.
 template <int T>
-__device__ void phase_bbox(const BatchArgs &A, uint32_t base, uint32_t n, BatchSmem<T> &S) {
+__device__ void phase_bbox(const BatchArgs &A, ClusterTeam &team, uint32_t base, uint32_t n,
+                           BatchCtl *ctl, BatchShared<T> &S) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float4 a = make_float4(FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX);
     bool bad = false;
-    for (uint32_t i = threadIdx.x; i < n; i += T) {
+    for (uint32_t i = (uint32_t)(team.rank * T) + threadIdx.x; i < n; i += (uint32_t)team.size * T) {
         const float2 p = A.pos[base + i];
         a = make_float4(fminf(a.x, p.x), fmaxf(a.y, p.x), fminf(a.z, p.y), fmaxf(a.w, p.y));
         bad |= !(isfinite(p.x) && isfinite(p.y));
     }
-    // a NaN or infinite position stops this graph's iterations
-    if (__any_sync(kFullMask, bad) && lane == 0) atomicOr(&S.err, kErrNonFinite);
+    if (__any_sync(kFullMask, bad) && lane == 0) ctl->bad = 1;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         a.x = fminf(a.x, __shfl_xor_sync(kFullMask, a.x, o));
@@ -240,6 +201,15 @@ __device__ void phase_bbox(const BatchArgs &A, uint32_t base, uint32_t n, BatchS
             const float4 c = S.wbox[w];
             b = make_float4(fminf(b.x, c.x), fmaxf(b.y, c.y), fminf(b.z, c.z), fmaxf(b.w, c.w));
         }
+        ctl->box[team.rank] = b;
+    }
+    team.sync();
+    if (threadIdx.x == 0) {
+        float4 b = ctl->box[0];
+        for (int r = 1; r < team.size; ++r) {
+            const float4 c = ctl->box[r];
+            b = make_float4(fminf(b.x, c.x), fmaxf(b.y, c.y), fminf(b.z, c.z), fmaxf(b.w, c.w));
+        }
         S.radius = fmaxf(b.y - b.x, b.w - b.z) * 0.5f;
         S.rx = (b.x + b.y) * 0.5f;
         S.ry = (b.z + b.w) * 0.5f;
@@ -247,326 +217,44 @@ __device__ void phase_bbox(const BatchArgs &A, uint32_t base, uint32_t n, BatchS
     __syncthreads();
 }
 
-// One stable LSD pass over the graph's n keys in chunks of T x kBRounds: digit
-// histogram, bases, then per chunk a ballot ranking per warp and offsets
-// across warps.
+// The walk over this graph's tree, the total force, swing and traction per
+// group of 32 bodies.
 template <int T>
-__device__ void sort_pass(int pass, uint32_t n, const uint64_t *kin, const uint32_t *vin,
-                          uint64_t *kout, uint32_t *vout, BatchSmem<T> &S) {
-    constexpr int kW = T / kWarp, kChunk = T * kBRounds;
-    constexpr int kQ = T / 256;  // threads per digit in the cross-warp offsets
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int shift = 8 * pass;
-    const unsigned lt = (1u << lane) - 1u;
-    if (threadIdx.x < 256) S.base[threadIdx.x] = 0;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += T)
-        atomicAdd(&S.base[(uint32_t)(kin[i] >> shift) & 255u], 1u);
-    __syncthreads();
-    if (threadIdx.x < 256) {  // exclusive scan of the 256 counts (warps 0..7)
-        const uint32_t c = S.base[threadIdx.x];
-        uint32_t inc = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(kFullMask, inc, o);
-            if (lane >= o) inc += t;
-        }
-        if (lane == 31) S.coff[wid] = inc;
-        __syncwarp();
-        S.qsum[0][threadIdx.x] = inc - c;
-    }
-    __syncthreads();
-    if (threadIdx.x < 256) {
-        uint32_t b = 0;
-        for (int w = 0; w < wid; ++w) b += S.coff[w];
-        S.base[threadIdx.x] = S.qsum[0][threadIdx.x] + b;
-    }
-    __syncthreads();
-    for (uint32_t c0 = 0; c0 < n; c0 += kChunk) {
-        const uint32_t w0 = c0 + (uint32_t)wid * (kChunk / kW);
-        uint64_t k[kBRounds];
-        uint32_t v[kBRounds], rank[kBRounds];
-#pragma unroll
-        for (int r = 0; r < kBRounds; ++r) {
-            const uint32_t idx = w0 + (uint32_t)(r * 32 + lane);
-            k[r] = idx < n ? kin[idx] : 0ull;
-            v[r] = idx < n ? vin[idx] : 0u;
-        }
-        for (int j = threadIdx.x; j < kW * 256; j += T) (&S.whist[0][0])[j] = 0;
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kBRounds; ++r) {
-            const bool valid = w0 + (uint32_t)(r * 32 + lane) < n;
-            const uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
-            unsigned peers = __ballot_sync(kFullMask, valid);
-            if (!valid) peers = ~peers;
-#pragma unroll
-            for (int b = 0; b < 8; ++b) {
-                const bool bit = (d >> b) & 1u;
-                const unsigned m = __ballot_sync(kFullMask, bit);
-                peers &= bit ? m : ~m;
-            }
-            uint32_t before = 0;
-            if (valid) before = S.whist[wid][d];
-            rank[r] = before + __popc(peers & lt);
-            __syncwarp();
-            if (valid && (peers & lt) == 0) S.whist[wid][d] = before + __popc(peers);
-            __syncwarp();
-        }
-        __syncthreads();
-        // per digit: exclusive offsets across the warps, kQ threads per digit
-        // taking 8 warps each
-        const int dg = threadIdx.x & 255, qt = threadIdx.x >> 8;
-        {
-            uint32_t q = 0;
-#pragma unroll
-            for (int w = 0; w < 8; ++w) q += S.whist[qt * 8 + w][dg];
-            S.qsum[qt][dg] = q;
-        }
-        __syncthreads();
-        {
-            uint32_t run = 0, tot = 0;
-#pragma unroll
-            for (int q = 0; q < kQ; ++q) {
-                const uint32_t c = S.qsum[q][dg];
-                if (q < qt) run += c;
-                tot += c;
-            }
-            run += S.base[dg];
-#pragma unroll
-            for (int w = 0; w < 8; ++w) {
-                const uint32_t c = S.whist[qt * 8 + w][dg];
-                S.whist[qt * 8 + w][dg] = run;
-                run += c;
-            }
-            if (qt == 0) S.coff[dg] = tot;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kBRounds; ++r) {
-            if (w0 + (uint32_t)(r * 32 + lane) < n) {
-                const uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
-                const uint32_t out = S.whist[wid][d] + rank[r];
-                kout[out] = k[r];
-                vout[out] = v[r];
-            }
-        }
-        if (threadIdx.x < 256) S.base[threadIdx.x] += S.coff[threadIdx.x];
-        __syncthreads();
-    }
-}
-
-// Keys from the positions, the sort passes (ending in keys0/vals0) and the
-// ordering of equal-key runs; returns with S.poison set if exactly
-// coincident bodies were found (perturb = 0) or after scaling them (1).
-// With first = 2 or 4 the sort skips its lowest 2 or 4 digits (after a tree
-// no deeper than level 22 or 14, so the digits it sorts reach two levels
-// deeper), and each run of keys equal in the digits it sorted is then
-// ordered by the full key, stably: exactly the order of the full sort (the
-// rule of the single-graph engine's k_fix_low).  A run longer than kBMaxRun
-// sorts the graph again on every digit.
-template <int T>
-__device__ void phase_keys_sort(const BatchArgs &A, uint32_t base, uint32_t n, char *slot,
-                                BatchSmem<T> &S, int perturb, int first = 0) {
-    uint64_t *k0 = slot_ptr<uint64_t>(slot, A.L.keys0), *k1 = slot_ptr<uint64_t>(slot, A.L.keys1);
-    uint32_t *v0 = slot_ptr<uint32_t>(slot, A.L.vals0), *v1 = slot_ptr<uint32_t>(slot, A.L.vals1);
-    const float rx = S.rx, ry = S.ry, rr = S.radius;
-    for (uint32_t i = threadIdx.x; i < n; i += T) {
-        const float2 p = A.pos[base + i];
-        k0[i] = morton_key(p.x, p.y, rx, ry, rr);
-        v0[i] = i;
-    }
-    if (threadIdx.x == 0) S.resort = 0;
-    __syncthreads();
-    for (int pass = first; pass < 8; pass += 2) {
-        sort_pass(pass, n, k0, v0, k1, v1, S);
-        sort_pass(pass + 1, n, k1, v1, k0, v0, S);
-    }
-    if (first > 0) {
-        const int low = 8 * first;
-        for (uint32_t k = threadIdx.x; k + 1 < n; k += T) {
-            const uint64_t hk = k0[k] >> low;
-            if ((k0[k + 1] >> low) != hk || (k > 0 && (k0[k - 1] >> low) == hk)) continue;
-            uint32_t len = 2;
-            while (k + len < n && (k0[k + len] >> low) == hk && len <= (uint32_t)kBMaxRun) ++len;
-            if (len > (uint32_t)kBMaxRun) {
-                S.resort = 1;
-                continue;
-            }
-            uint64_t *kr = k0 + k;
-            uint32_t *vr = v0 + k;
-            for (uint32_t a = 1; a < len; ++a) {  // insertion sort, stable
-                const uint64_t ka = kr[a];
-                const uint32_t va = vr[a];
-                int j = (int)a - 1;
-                while (j >= 0 && kr[j] > ka) {
-                    kr[j + 1] = kr[j];
-                    vr[j + 1] = vr[j];
-                    --j;
-                }
-                kr[j + 1] = ka;
-                vr[j + 1] = va;
-            }
-        }
-        __syncthreads();
-        // every digit, from the order the partial sort left: equal keys keep
-        // their input order through both, so this is the full sort's order
-        if (S.resort)
-            for (int pass = 0; pass < 8; pass += 2) {
-                sort_pass(pass, n, k0, v0, k1, v1, S);
-                sort_pass(pass + 1, n, k1, v1, k0, v0, S);
-            }
-    }
-    for (uint32_t k = threadIdx.x; k + 1 < n; k += T) {
-        if (k0[k + 1] != k0[k] || (k > 0 && k0[k - 1] == k0[k])) continue;
-        fix_run((int)k, (int)n, k0, v0, A.pos + base, nullptr, rx, ry, rr, &S.err, &S.poison,
-                perturb);
-    }
-    __syncthreads();
-}
-
-// Tree count: L[k], preorder indices, owners and the exact prefix sums.
-template <int T>
-__device__ void phase_count(const BatchArgs &A, uint32_t base, uint32_t n, char *slot,
-                            BatchSmem<T> &S) {
-    const uint64_t *keys = slot_ptr<uint64_t>(slot, A.L.keys0);
-    const uint32_t *vals = slot_ptr<uint32_t>(slot, A.L.vals0);
-    int8_t *lcp = slot_ptr<int8_t>(slot, A.L.lcp);
-    uint32_t *group = slot_ptr<uint32_t>(slot, A.L.group);
-    uint32_t *owner = slot_ptr<uint32_t>(slot, A.L.owner);
-    long long *pm = slot_ptr<long long>(slot, A.L.pm);
-    i128 *pxy = slot_ptr<i128>(slot, A.L.pxy);
-    const double scale = S.radius > 0.0f ? kFixedScale / (double)S.radius : 1.0;
-    const float rx = S.rx, ry = S.ry;
-    const uint32_t cap = A.L.cap;
-    NodeSums carry{0, 0, 0, 0};
-    int lmax = 0;  // this thread's deepest shared-digit count: the tree's depth
-    if (threadIdx.x == 0) S.maxlev = 0;
-    for (uint32_t c0 = 0; c0 < n; c0 += T) {
-        const uint32_t k = c0 + threadIdx.x;
-        NodeSums v{0, 0, 0, 0};
-        long long im = 0, qx = 0, qy = 0;
-        int c = 0;
-        if (k < n) {
-            const int Lk = lcp_at(keys, (int)n, (int)k), Lkm1 = lcp_at(keys, (int)n, (int)k - 1);
-            lmax = Lk > lmax ? Lk : lmax;
-            lcp[k] = (int8_t)Lk;
-            c = cells_at((int)k, Lk, Lkm1);
-            const uint32_t i = vals[k];
-            const float2 p = A.pos[base + i];
-            im = (long long)A.mass[base + i];
-            qx = fixed_offset(p.x, rx, scale);
-            qy = fixed_offset(p.y, ry, scale);
-            v.g = (uint32_t)c + 1u;
-            v.m = im;
-            v.x = (i128)im * qx;
-            v.y = (i128)im * qy;
-        }
-        NodeSums total;
-        NodeSums ex = block_scan(v, S, &total);
-        sums_add(ex, carry);
-        if (k < n) {
-            group[k] = ex.g;
-            pm[k] = ex.m;
-            pxy[2 * (size_t)k] = ex.x;
-            pxy[2 * (size_t)k + 1] = ex.y;
-            for (uint32_t q = 0; q <= (uint32_t)c; ++q) {
-                const uint32_t idx = ex.g + q;
-                if (idx < cap) owner[idx] = (k << 6) | (q < (uint32_t)c ? q : 63u);
-            }
-        }
-        sums_add(carry, total);
-    }
-    atomicMax(&S.maxlev, lmax);
-    if (threadIdx.x == 0) {
-        pm[n] = carry.m;
-        pxy[2 * (size_t)n] = carry.x;
-        pxy[2 * (size_t)n + 1] = carry.y;
-        S.total_nodes = carry.g;
-        if (carry.g > cap) S.err |= kErrTreeTooLarge;
-    }
-    __syncthreads();
-}
-
-// Every node of the tree once (k_emit's rule, one thread per node).
-template <int T>
-__device__ void phase_emit(const BatchArgs &A, uint32_t base, uint32_t n, char *slot,
-                           BatchSmem<T> &S) {
-    const uint64_t *keys = slot_ptr<uint64_t>(slot, A.L.keys0);
-    const uint32_t *vals = slot_ptr<uint32_t>(slot, A.L.vals0);
-    const int8_t *lcp = slot_ptr<int8_t>(slot, A.L.lcp);
-    const uint32_t *group = slot_ptr<uint32_t>(slot, A.L.group);
-    const uint32_t *owner = slot_ptr<uint32_t>(slot, A.L.owner);
-    const long long *pm = slot_ptr<long long>(slot, A.L.pm);
-    const i128 *pxy = slot_ptr<i128>(slot, A.L.pxy);
-    float4 *nodes = slot_ptr<float4>(slot, A.L.nodes);
-    uint32_t *body_node = slot_ptr<uint32_t>(slot, A.L.body_node);
-    const double inv_scale = S.radius > 0.0f ? (double)S.radius / kFixedScale : 1.0;
-    const double rx = S.rx, ry = S.ry;
-    const uint32_t total = S.total_nodes;
-    for (uint32_t g = threadIdx.x; g < total; g += T) {
-        const uint32_t w = owner[g];
-        const int k = (int)(w >> 6), q = (int)(w & 63u);
-        if (q == 63) {
-            const uint32_t i = vals[k];
-            const float2 p = A.pos[base + i];
-            nodes[g] = make_float4(p.x, p.y, A.mass[base + i], make_meta(g + 1, kBodyLevel));
-            body_node[k] = g;
-            continue;
-        }
-        const int lvl = (k == 0 ? 0 : load_lcp(lcp, (int)n, k - 1) + 1) + q;
-        const int b = lvl == 0 ? (int)n - 1 : find_end(keys, lcp, (int)n, k, lvl);
-        const uint32_t next = body_index(lcp, group, (int)n, b) + 1;
-        const double cm = (double)(pm[b + 1] - pm[k]);
-        const double sx = i128_to_double(pxy[2 * (size_t)(b + 1)] - pxy[2 * (size_t)k]);
-        const double sy = i128_to_double(pxy[2 * (size_t)(b + 1) + 1] - pxy[2 * (size_t)k + 1]);
-        nodes[g] = make_float4((float)(rx + sx / cm * inv_scale), (float)(ry + sy / cm * inv_scale),
-                               (float)cm, make_meta(next, lvl));
-    }
-    __syncthreads();
-}
-
-// The warp-vote walk of k_traverse over this graph's tree, the total force,
-// swing and traction per group of 32 bodies, then (thread 0) the speed rule.
-template <int T>
-__device__ void phase_traverse(const BatchArgs &A, uint32_t base, uint32_t n, char *slot,
-                               BatchSmem<T> &S) {
+__device__ void phase_traverse(const BatchArgs &A, const ClusterTeam &team, uint32_t base,
+                               uint32_t n, char *slot, BatchCtl *ctl, BatchShared<T> &S,
+                               WalkWarp<false, false> *walk) {
     const float4 *nodes = slot_ptr<float4>(slot, A.L.nodes);
-    const uint32_t *body_node = slot_ptr<uint32_t>(slot, A.L.body_node);
-    const uint32_t *vals = slot_ptr<uint32_t>(slot, A.L.vals0);
+    const float4 *sbody = slot_ptr<float4>(slot, A.L.sbody);
     const float2 *fa = slot_ptr<float2>(slot, A.L.fa);
     float2 *f = slot_ptr<float2>(slot, A.L.f);
     float2 *gpart = slot_ptr<float2>(slot, A.L.gpart);
-    const int lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) {
-        walk_thresholds(S.radius, A.prm, S.dq);
-        S.ticket = 0;
-    }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (threadIdx.x == 0) walk_thresholds(S.radius, A.prm, S.dq);
     __syncthreads();
-    const uint32_t end = S.total_nodes;
+    const uint32_t end = *(volatile uint32_t *)&ctl->tree_nodes;
     const int ngroups = (int)((n + 31) >> 5);
-    for (;;) {
-        int w = 0;
-        if (lane == 0) w = atomicAdd(&S.ticket, 1);
-        w = __shfl_sync(kFullMask, w, 0);
-        if (w >= ngroups) break;
+    // a warp's first group spreads the groups over the blocks, the others come
+    // from the ticket
+    int w = wid * team.size + team.rank;
+    while (w < ngroups) {
         const int k = w * 32 + lane;
         const bool active = k < (int)n;
-        const float4 me = nodes[body_node[active ? k : (int)n - 1]];
+        const float4 me = sbody[active ? k : (int)n - 1];
         const float px = active ? me.x : 1e30f, py = active ? me.y : 1e30f;
         auto none = [](bool, const float4 &, float, uint32_t) {};
-        WalkWarp<false, false> &W = S.walk[threadIdx.x >> 5];
         const float2 a =
             A.prm.epssq >= FLT_MIN
-                ? walk_group<false, false, false, true>(W, S.dq, nodes, nullptr, nullptr, nullptr,
-                                                        end, px, py, 0.0f, A.prm.epssq, none)
-                : walk_group<false, false, false, false>(W, S.dq, nodes, nullptr, nullptr, nullptr,
-                                                         end, px, py, 0.0f, A.prm.epssq, none);
+                ? walk_group<false, false, false, true>(walk[wid], S.dq, nodes, nullptr, nullptr,
+                                                        nullptr, end, px, py, 0.0f, A.prm.epssq,
+                                                        none)
+                : walk_group<false, false, false, false>(walk[wid], S.dq, nodes, nullptr, nullptr,
+                                                         nullptr, end, px, py, 0.0f, A.prm.epssq,
+                                                         none);
         const float kmi = A.prm.k_r * me.z;
         const float ax = __fmul_rn(a.x, kmi), ay = __fmul_rn(a.y, kmi);
         float sw = 0.0f, tr = 0.0f;
         if (active) {
-            const uint32_t i = vals[k];
+            const uint32_t i = __float_as_uint(me.w);
             const float2 g = fa[i], fp = A.fprev[base + i];
             const float fx = g.x + ax, fy = g.y + ay;
             f[i] = make_float2(fx, fy);
@@ -582,10 +270,20 @@ __device__ void phase_traverse(const BatchArgs &A, uint32_t base, uint32_t n, ch
             sw += __shfl_xor_sync(kFullMask, sw, o);
             tr += __shfl_xor_sync(kFullMask, tr, o);
         }
-        if (lane == 0) gpart[w] = make_float2(sw, tr);
+        if (lane == 0) {
+            gpart[w] = make_float2(sw, tr);
+            w = team.size * (T / kWarp) + atomicAdd(&ctl->ticket, 1);
+        }
+        w = __shfl_sync(kFullMask, w, 0);
     }
-    __syncthreads();
-    // fixed-order sum of the group partials, then the speed rule
+}
+
+// The speed rule from the group partials, summed in a fixed order (by each
+// block for itself).
+template <int T>
+__device__ void phase_speed(const BatchArgs &A, uint32_t n, char *slot, BatchShared<T> &S) {
+    const float2 *gpart = slot_ptr<float2>(slot, A.L.gpart);
+    const int lane = threadIdx.x & 31, ngroups = (int)((n + 31) >> 5);
     if (threadIdx.x < 32) {
         float sw = 0.0f, tr = 0.0f;
         for (int w = lane; w < ngroups; w += 32) {
@@ -610,11 +308,10 @@ __device__ void phase_traverse(const BatchArgs &A, uint32_t base, uint32_t n, ch
 
 // Displacement (DisplacementKernel, src/RPFA2Kernels.cu:223-251).
 template <int T>
-__device__ void phase_displace(const BatchArgs &A, uint32_t base, uint32_t n, char *slot,
-                               BatchSmem<T> &S) {
+__device__ void phase_displace(const BatchArgs &A, const ClusterTeam &team, uint32_t base,
+                               uint32_t n, char *slot, float gs) {
     const float2 *f = slot_ptr<float2>(slot, A.L.f);
-    const float gs = S.gs;
-    for (uint32_t i = threadIdx.x; i < n; i += T) {
+    for (uint32_t i = (uint32_t)(team.rank * T) + threadIdx.x; i < n; i += (uint32_t)team.size * T) {
         const float2 fi = f[i], fp = A.fprev[base + i];
         const float factor = displacement_factor(fi, fp, gs);
         float2 p = A.pos[base + i];
@@ -623,7 +320,6 @@ __device__ void phase_displace(const BatchArgs &A, uint32_t base, uint32_t n, ch
         A.pos[base + i] = p;
         A.fprev[base + i] = fi;
     }
-    __syncthreads();
 }
 
 // 1024 threads per SM, 64 registers a thread: a warp's walk has 32 loads in
@@ -632,71 +328,129 @@ __device__ void phase_displace(const BatchArgs &A, uint32_t base, uint32_t n, ch
 // CTAs above), 1024, 1536 and 2048 threads per SM: 1.74, 1.74 and 1.99 ms an
 // iteration; on 96 graphs of 50 to 600 nodes 90, 103 and 112 us.
 constexpr int kBatchThreadsPerSm = 1024;
+
+// Launched in clusters of the team's size.
 template <int T, bool LINLOG>
 __global__ void __launch_bounds__(T, kBatchThreadsPerSm / T) k_batch(BatchArgs A) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    BatchSmem<T> &S = *reinterpret_cast<BatchSmem<T> *>(smem_raw);
-    char *slot = A.slots + (size_t)blockIdx.x * A.L.bytes;
+    extern __shared__ __align__(64) unsigned char smem_raw[];
+    BatchShared<T> &S = *reinterpret_cast<BatchShared<T> *>(smem_raw);
+    unsigned char *turns = smem_raw + kBatchHead<T>;
+    BuildSmem<T> &B = *reinterpret_cast<BuildSmem<T> *>(turns);
+    auto *walk = reinterpret_cast<WalkWarp<false, false> *>(turns);
+    uint32_t crank, csize;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
+    ClusterTeam team{(int)crank, (int)csize};
+    char *slot = A.slots + (size_t)(blockIdx.x / csize) * A.L.bytes;
+    BatchCtl *ctl = slot_ptr<BatchCtl>(slot, A.L.ctl);
     float2 *fa = slot_ptr<float2>(slot, A.L.fa);
+    const bool leader = team.rank == 0 && threadIdx.x == 0;
+    const int tid0 = team.rank * T + (int)threadIdx.x, stride = team.size * T;
+    auto flag = [](const int *p) { return *(const volatile int *)p; };
     for (;;) {
-        if (threadIdx.x == 0) S.graph = (int)atomicAdd(A.queue, 1u);
-        __syncthreads();
-        const int qi = S.graph;
+        if (leader) ctl->graph = (int)atomicAdd(A.queue, 1u);
+        team.sync();
+        const int qi = flag(&ctl->graph);
         if (qi >= A.num_graphs) break;
         const int gi = (int)A.order[qi];
         const BatchGraph G = A.graphs[gi];
         const uint32_t base = G.node_base, n = G.n;
+        const BatchSpeed sp = A.speed[gi];
         if (threadIdx.x == 0) {
-            const BatchSpeed sp = A.speed[gi];
             S.gs = sp.global_speed;
             S.se = sp.speed_efficiency;
-            S.err = sp.err;
-            S.poison = 0;
         }
-        __syncthreads();
-        int rounds = 0;
-        int first = 0;  // low digits the next sort skips, from the last tree's depth
-        for (int it = 0; it < A.iters && n > 0; ++it) {
-            if (S.err) break;
-            phase_attract<T, LINLOG>(A, base, n, fa);
-            phase_bbox(A, base, n, S);
-            if (S.err) break;
-            phase_keys_sort(A, base, n, slot, S, 0, first);
+        if (leader) {
+            ctl->err = sp.err;
+            ctl->poison = 0;
+            ctl->bad = 0;
+            ctl->resorts = 0;
+            for (int l = 0; l < kCellLevels; ++l) ctl->cells[l] = 0;  // no last tree
+        }
+        BuildArgs T_{};
+        T_.n = (int)n;
+        T_.pos = A.pos + base;
+        T_.mass = A.mass + base;
+        T_.ref_of = nullptr;
+        T_.keys[0] = slot_ptr<uint64_t>(slot, A.L.keys0);
+        T_.keys[1] = slot_ptr<uint64_t>(slot, A.L.keys1);
+        T_.vals[0] = slot_ptr<uint32_t>(slot, A.L.vals0);
+        T_.vals[1] = slot_ptr<uint32_t>(slot, A.L.vals1);
+        T_.sbody = slot_ptr<float4>(slot, A.L.sbody);
+        T_.lcp = slot_ptr<uint8_t>(slot, A.L.lcp);
+        T_.rowmin = slot_ptr<uint8_t>(slot, A.L.rowmin);
+        T_.tilemin = slot_ptr<uint8_t>(slot, A.L.tilemin);
+        T_.defer = slot_ptr<uint32_t>(slot, A.L.defer);
+        T_.group = slot_ptr<uint32_t>(slot, A.L.group);
+        T_.body_node = slot_ptr<uint32_t>(slot, A.L.body_node);
+        T_.owner = slot_ptr<uint32_t>(slot, A.L.owner);
+        T_.nodes = slot_ptr<float4>(slot, A.L.nodes);
+        T_.capacity = A.L.cap;
+        T_.pm = slot_ptr<long long>(slot, A.L.pm);
+        T_.pxy = slot_ptr<i128>(slot, A.L.pxy);
+        T_.counts = slot_ptr<uint32_t>(slot, A.L.counts);
+        T_.totals = slot_ptr<NodeSums>(slot, A.L.totals);
+        T_.err = &ctl->err;
+        T_.poison = &ctl->poison;
+        T_.resort = &ctl->resort;
+        T_.resorts = &ctl->resorts;
+        T_.deep = &ctl->deep;
+        T_.cells = ctl->cells;
+        T_.tree_nodes = &ctl->tree_nodes;
+        T_.max_level = &ctl->max_level;
+        team.sync();
+        int rounds = 0, err = flag(&ctl->err);
+        for (int it = 0; it < A.iters && n > 0 && !err; ++it) {
+            phase_attract<T, LINLOG>(A, team, base, n, fa);
+            phase_bbox(A, team, base, n, ctl, S);
+            // a NaN or infinite position stops this graph's iterations
+            if (flag(&ctl->bad)) {
+                err = kErrNonFinite;
+                break;
+            }
+            T_.rootx = S.rx;
+            T_.rooty = S.ry;
+            T_.radius = S.radius;
             // Exactly coincident bodies: scale the later ones by .99 (the
             // reference's re-insertion, src/RPBHKernels.cu:271-278) and build
             // again, keeping gravity, attraction and the box of before.
-            rounds = 0;
-            while (S.poison && !S.err) {
-                if (++rounds > 64) {
-                    if (threadIdx.x == 0) S.err |= kErrPoisonRounds;
-                    __syncthreads();
+            for (rounds = 0;; ++rounds) {
+                if (leader) ctl->ticket = 0;
+                build_tree(T_, team, B, A.chunk);
+                team.sync();
+                err = flag(&ctl->err);
+                if (err || !flag(&ctl->poison)) break;
+                if (rounds >= 64) {
+                    err = kErrPoisonRounds;
                     break;
                 }
-                __syncthreads();
-                if (threadIdx.x == 0) S.poison = 0;
-                phase_keys_sort(A, base, n, slot, S, 1);  // scales, poison stays 0
-                phase_keys_sort(A, base, n, slot, S, 0);  // sorts the scaled positions
+                for (int k = tid0; k + 1 < (int)n; k += stride)
+                    if (T_.keys[0][k + 1] == T_.keys[0][k] &&
+                        !(k > 0 && T_.keys[0][k - 1] == T_.keys[0][k]))
+                        fix_run(k, (int)n, T_.keys[0], T_.vals[0], T_.pos, nullptr, S.rx, S.ry,
+                                S.radius, &ctl->err, &ctl->poison, 1);
+                team.sync();
+                if (leader) ctl->poison = 0;
+                team.sync();
             }
-            if (S.err) break;
-            phase_count(A, base, n, slot, S);
-            if (S.err) break;
-            first = S.maxlev <= kLevels - 18 ? 4 : (S.maxlev <= kLevels - 10 ? 2 : 0);
-            phase_emit(A, base, n, slot, S);
-            phase_traverse(A, base, n, slot, S);
-            phase_displace(A, base, n, slot, S);
+            if (err) break;
+            phase_traverse(A, team, base, n, slot, ctl, S, walk);
+            team.sync();
+            phase_speed(A, n, slot, S);
+            phase_displace<T>(A, team, base, n, slot, S.gs);
+            team.sync();
         }
         // the body order of the last iteration, graph-local ids
-        const uint32_t *vals = slot_ptr<uint32_t>(slot, A.L.vals0);
-        for (uint32_t k = threadIdx.x; k < n; k += T) A.sortd[base + k] = vals[k];
-        if (threadIdx.x == 0) {
-            BatchSpeed sp;
-            sp.global_speed = S.gs;
-            sp.speed_efficiency = S.se;
-            sp.err = S.err;
-            sp.perturb_rounds = rounds;
-            A.speed[gi] = sp;
+        for (int k = tid0; k < (int)n; k += stride) A.sortd[base + k] = T_.vals[0][k];
+        if (leader) {
+            BatchSpeed out;
+            out.global_speed = S.gs;
+            out.speed_efficiency = S.se;
+            out.err = err;
+            out.perturb_rounds = rounds;
+            A.speed[gi] = out;
         }
-        __syncthreads();
+        team.sync();
     }
 }
 
@@ -707,9 +461,9 @@ __global__ void k_clear_errors(int n, BatchSpeed *__restrict speed) {
 
 size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-SlotLayout make_layout(uint32_t nmax) {
+SlotLayout make_layout(uint32_t nmax, int team) {
     SlotLayout L;
-    const uint64_t cap64 = 33ull * nmax + 64;
+    const uint64_t cap64 = 33ull * nmax + 64, rows = (nmax + 31) / 32;
     L.cap = (uint32_t)cap64;
     size_t o = 0;
     auto take = [&](size_t bytes) {
@@ -717,20 +471,27 @@ SlotLayout make_layout(uint32_t nmax) {
         o = up256(o + bytes);
         return at;
     };
+    L.ctl = take(sizeof(BatchCtl));
     L.keys0 = take(8ull * nmax);
     L.keys1 = take(8ull * nmax);
     L.vals0 = take(4ull * nmax);
     L.vals1 = take(4ull * nmax);
-    L.lcp = take(1ull * nmax);
+    L.sbody = take(16ull * nmax);
+    L.lcp = take(pad64(nmax));
+    L.rowmin = take(pad64(rows));
+    L.tilemin = take(pad64((size_t)team));
+    L.defer = take(4ull * (kLevels + 1) * rows);
     L.group = take(4ull * nmax);
     L.body_node = take(4ull * nmax);
     L.owner = take(4ull * cap64);
     L.nodes = take(16ull * (cap64 + 1));
     L.pm = take(8ull * (nmax + 1));
     L.pxy = take(32ull * (nmax + 1));
+    L.counts = take(4ull * build_counts(team));
+    L.totals = take(build_totals_bytes(team));
     L.fa = take(8ull * nmax);
     L.f = take(8ull * nmax);
-    L.gpart = take(8ull * ((nmax + 31) / 32));
+    L.gpart = take(8ull * rows);
     L.bytes = o;
     return L;
 }
@@ -742,14 +503,29 @@ SlotLayout make_layout(uint32_t nmax) {
 using namespace fa2;
 
 // One size class of the batch: its graphs (a slice of the queue order), the
-// CTA size that runs them, and its grid with one scratch slot per CTA.
+// teams that run them, and its grid with one scratch slot per team.
 struct BatchClass {
     BatchArgs args{};
-    int threads = 0;        // 0: the class is empty
-    int grid = 0;
+    int threads = 0;        // per block; 0: the class is empty
+    int team = 1;           // blocks per graph, one cluster
+    int grid = 0;           // teams
+    size_t smem = 0;
     void *slots = nullptr;  // grid x args.L.bytes
     size_t slot_cap = 0;    // bytes allocated at slots
 };
+
+// A split's two sides, each of one class or one per team size.
+constexpr int kMaxClasses = 6;
+
+// How many 512-thread blocks (one cluster) run a graph of at most so many
+// nodes.  Measured on 512 graphs of 50 to 20,000 nodes: 1.16 ms an iteration;
+// teams of 4 already from 1024 nodes and of 8 from 4096 1.24 ms, of 4 only
+// from 4096 nodes 1.35 ms, of 2 instead of 4 1.28 ms.
+struct BatchTeam {
+    uint32_t upto;
+    int team;
+};
+constexpr BatchTeam kTeams[3] = {{2048, 1}, {8192, 4}, {kBatchMaxNodes, 8}};
 
 struct fa2_batch {
     int device = 0;
@@ -765,16 +541,18 @@ struct fa2_batch {
     BatchArgs args{};             // the fields every class shares
     uint32_t *d_order = nullptr;  // the queue order of the current classes
     unsigned *queues = nullptr;   // one ticket counter per class
-    // Graphs of at most `split` nodes (class 0) run on CTAs of `small_threads`
-    // threads, the others (class 1) on CTAs of `large_threads`.
+    // Graphs of at most `split` nodes run on `small_threads`, the others on
+    // `large_threads`: 256 is one block of 256 threads per graph, 512 and 1024
+    // are blocks of 512 threads, one or a cluster of them by the graph's size
+    // (kTeams).  The classes that makes, small graphs first.
     uint32_t split = 0;
     int small_threads = 256, large_threads = 1024;
-    BatchClass cls[2];
+    std::vector<BatchClass> cls;
     // the launch of one step call, captured for its iteration count
     cudaGraphExec_t exec = nullptr;
     int exec_iters = -1;
-    cudaStream_t stream = nullptr, side = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr, evFork = nullptr, evJoin = nullptr;
+    cudaStream_t stream = nullptr, side[kMaxClasses] = {};
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, evFork = nullptr, evJoin[kMaxClasses] = {};
 };
 
 namespace {
@@ -811,61 +589,107 @@ void bfree(fa2_batch *b) {
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     if (b->evFork) cudaEventDestroy(b->evFork);
-    if (b->evJoin) cudaEventDestroy(b->evJoin);
+    for (cudaEvent_t e : b->evJoin)
+        if (e) cudaEventDestroy(e);
     if (b->stream) cudaStreamDestroy(b->stream);
-    if (b->side) cudaStreamDestroy(b->side);
+    for (cudaStream_t t : b->side)
+        if (t) cudaStreamDestroy(t);
     for (BatchClass &c : b->cls)
         if (c.slots) cudaFree(c.slots);
     for (void *p : b->allocs) cudaFree(p);
     b->allocs.clear();
 }
 
-template <int T>
-int occupancy() {
-    int a = 0, c = 0;
-    const int bytes = (int)sizeof(BatchSmem<T>);
-    cudaFuncSetAttribute(k_batch<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_batch<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_batch<T, false>, T, bytes);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_batch<T, true>, T, bytes);
-    return std::max(1, std::min(a, c));
-}
-
-int occupancy_for(int threads) {
-    switch (threads) {
-        case 256: return occupancy<256>();
-        case 512: return occupancy<512>();
-        default: return occupancy<1024>();
+// The launch of a class on a stream (or, with teams, only how many of its
+// teams the GPU holds at once).
+template <int T, bool LINLOG>
+int launch_class(const BatchClass &c, cudaStream_t s, int *teams) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)c.team;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(c.team * std::max(1, c.grid)));
+    cfg.blockDim = dim3(T);
+    cfg.dynamicSmemBytes = c.smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = c.team > 1 ? 1 : 0;
+    if (teams) {
+        // the most any class of this kernel asks for
+        BCK(cudaFuncSetAttribute(k_batch<T, LINLOG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)batch_smem_bytes<T>(T * kBuildRounds)));
+        if (c.team > 1)
+            return cuda_status_b(cudaOccupancyMaxActiveClusters(teams, k_batch<T, LINLOG>, &cfg));
+        int per_sm = 0;
+        BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<T, LINLOG>, T, c.smem));
+        *teams = per_sm * c.args.prm.nsm;
+        return FA2_OK;
     }
+    return cuda_status_b(cudaLaunchKernelEx(&cfg, k_batch<T, LINLOG>, c.args));
 }
 
-// Splits the graphs into the two classes, uploads the queue order (class 1
-// then class 0, each largest first) and sizes each class's grid and slots.
+int launch_class(const BatchClass &c, bool linlog, cudaStream_t s, int *teams) {
+    if (c.threads == 256)
+        return linlog ? launch_class<256, true>(c, s, teams) : launch_class<256, false>(c, s, teams);
+    return linlog ? launch_class<512, true>(c, s, teams) : launch_class<512, false>(c, s, teams);
+}
+
+// Splits the graphs into classes, uploads the queue order (class after class,
+// each largest first) and sizes each class's grid and slots.
 int configure(fa2_batch *b, uint32_t split, int small_threads, int large_threads) {
     drop_graph(b);  // the classes' grids and arguments are part of the graph
-    std::vector<uint32_t> big, small;
-    for (uint32_t g : b->order) (b->count[g] <= split ? small : big).push_back(g);
-    std::vector<uint32_t> q(big);
-    q.insert(q.end(), small.begin(), small.end());
+    // {largest graph of the class, threads per block, blocks per graph}
+    struct Kind {
+        uint32_t upto;
+        int threads, team;
+    };
+    std::vector<Kind> kinds;
+    auto add = [&](uint32_t upto, int threads) {
+        if (threads > 256)
+            for (const BatchTeam &k : kTeams)
+                kinds.push_back(Kind{std::min(upto, k.upto), 512, k.team});
+        else
+            kinds.push_back(Kind{upto, 256, 1});
+    };
+    if (split) add(split, small_threads);
+    add(kBatchMaxNodes, large_threads);
+    std::vector<std::vector<uint32_t>> members(kinds.size());
+    for (uint32_t g : b->order) {
+        // the first kind that takes it: the small side's come first
+        size_t k = 0;
+        while (b->count[g] > kinds[k].upto) ++k;
+        members[k].push_back(g);
+    }
+    std::vector<uint32_t> q;
+    for (const auto &m : members) q.insert(q.end(), m.begin(), m.end());
     if (!q.empty())
         BCK(cudaMemcpyAsync(b->d_order, q.data(), q.size() * 4, cudaMemcpyHostToDevice,
                             b->stream));
-    const std::vector<uint32_t> *members[2] = {&small, &big};
-    const uint32_t first[2] = {(uint32_t)big.size(), 0u};
-    const int threads[2] = {small_threads, large_threads};
-    for (int k = 0; k < 2; ++k) {
+    b->cls.resize(std::max(b->cls.size(), kinds.size()));
+    for (BatchClass &c : b->cls) c.threads = 0;
+    uint32_t first = 0;
+    for (size_t k = 0; k < kinds.size(); ++k) {
+        const std::vector<uint32_t> &m = members[k];
+        if (m.empty()) continue;
         BatchClass &c = b->cls[k];
-        const std::vector<uint32_t> &m = *members[k];
         c.args = b->args;
-        c.threads = m.empty() ? 0 : threads[k];
-        if (!c.threads) continue;
+        c.threads = kinds[k].threads;
+        c.team = kinds[k].team;
         uint32_t nmax = 1;
         for (uint32_t g : m) nmax = std::max(nmax, b->count[g]);
-        c.args.order = b->d_order + first[k];
+        c.args.order = b->d_order + first;
+        first += (uint32_t)m.size();
         c.args.num_graphs = (int)m.size();
         c.args.queue = b->queues + k;
-        c.args.L = make_layout(nmax);
-        c.grid = std::max(1, std::min<int>(b->nsm * occupancy_for(c.threads), (int)m.size()));
+        c.args.L = make_layout(nmax, c.team);
+        c.args.chunk = build_chunk(build_tile((int)nmax, c.team), c.threads);
+        c.smem = c.threads == 256 ? batch_smem_bytes<256>(c.args.chunk)
+                                  : batch_smem_bytes<512>(c.args.chunk);
+        int teams = 0;
+        const int s = launch_class(c, b->kp.linlog != 0, b->stream, &teams);
+        if (s) return s;
+        c.grid = std::max(1, std::min<int>(teams, (int)m.size()));
         const size_t need = c.args.L.bytes * (size_t)c.grid;
         if (need > c.slot_cap) {
             if (c.slots) cudaFree(c.slots);
@@ -883,38 +707,28 @@ int configure(fa2_batch *b, uint32_t split, int small_threads, int large_threads
     return FA2_OK;
 }
 
-template <bool LINLOG>
-void launch_class(const BatchClass &c, cudaStream_t s) {
-    switch (c.threads) {
-        case 256: k_batch<256, LINLOG><<<c.grid, 256, sizeof(BatchSmem<256>), s>>>(c.args); break;
-        case 512: k_batch<512, LINLOG><<<c.grid, 512, sizeof(BatchSmem<512>), s>>>(c.args); break;
-        default: k_batch<1024, LINLOG><<<c.grid, 1024, sizeof(BatchSmem<1024>), s>>>(c.args); break;
-    }
-}
-
-// Both classes at once: class 1 (large graphs) on the batch stream, class 0
-// on a second stream, joined back into the batch stream.
+// All classes at once, the largest graphs' first: that one on the batch
+// stream, the others on side streams joined back into it.
 int launch_batch(fa2_batch *b, int iters) {
-    BCK(cudaMemsetAsync(b->queues, 0, 2 * sizeof(unsigned), b->stream));
-    const bool both = b->cls[0].threads && b->cls[1].threads;
-    if (both) {
-        BCK(cudaEventRecord(b->evFork, b->stream));
-        BCK(cudaStreamWaitEvent(b->side, b->evFork, 0));
-    }
-    for (int k = 1; k >= 0; --k) {
+    BCK(cudaMemsetAsync(b->queues, 0, kMaxClasses * sizeof(unsigned), b->stream));
+    BCK(cudaEventRecord(b->evFork, b->stream));
+    bool main = true;
+    for (int k = (int)b->cls.size() - 1; k >= 0; --k) {
         BatchClass &c = b->cls[k];
         if (!c.threads) continue;
         c.args.iters = iters;
-        cudaStream_t s = (both && k == 0) ? b->side : b->stream;
-        if (b->kp.linlog)
-            launch_class<true>(c, s);
-        else
-            launch_class<false>(c, s);
-        BCK(cudaGetLastError());
+        cudaStream_t t = main ? b->stream : b->side[k];
+        if (!main) BCK(cudaStreamWaitEvent(t, b->evFork, 0));
+        const int s = launch_class(c, b->kp.linlog != 0, t, nullptr);
+        if (s) return s;
+        if (!main) BCK(cudaEventRecord(b->evJoin[k], t));
+        main = false;
     }
-    if (both) {
-        BCK(cudaEventRecord(b->evJoin, b->side));
-        BCK(cudaStreamWaitEvent(b->stream, b->evJoin, 0));
+    bool first = true;
+    for (int k = (int)b->cls.size() - 1; k >= 0; --k) {
+        if (!b->cls[k].threads) continue;
+        if (!first) BCK(cudaStreamWaitEvent(b->stream, b->evJoin[k], 0));
+        first = false;
     }
     return FA2_OK;
 }
@@ -1087,7 +901,7 @@ fa2_batch *fa2_batch_create(uint32_t num_graphs, const fa2_graph_desc *graphs,
         (s = balloc(b, &A.speed, std::max<size_t>(num_graphs, 1))) ||
         (s = balloc(b, &A.f_tot, std::max<size_t>(N, 1))) ||
         (s = balloc(b, &A.f_ag, std::max<size_t>(N, 1))) ||
-        (s = balloc(b, &A.sortd, std::max<size_t>(N, 1))) || (s = balloc(b, &b->queues, 2)))
+        (s = balloc(b, &A.sortd, std::max<size_t>(N, 1))) || (s = balloc(b, &b->queues, kMaxClasses)))
         return fail(s);
     A.graphs = d_graphs;
     A.mass = d_mass;
@@ -1097,11 +911,13 @@ fa2_batch *fa2_batch_create(uint32_t num_graphs, const fa2_graph_desc *graphs,
     A.jitter_tolerance = prm->jitter_tolerance;
     A.k_s_max = prm->k_s_max;
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->evFork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->evJoin, cudaEventDisableTiming) != cudaSuccess)
+        cudaEventCreateWithFlags(&b->evFork, cudaEventDisableTiming) != cudaSuccess)
         return fail(FA2_ERR_CUDA);
+    for (int k = 0; k < kMaxClasses; ++k)
+        if (cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&b->evJoin[k], cudaEventDisableTiming) != cudaSuccess)
+            return fail(FA2_ERR_CUDA);
     std::vector<BatchSpeed> sp(num_graphs);
     for (auto &x : sp) x = BatchSpeed{1.0f, 1.0f, 0, 0};  // src/RPFA2Kernels.cu:30-31
     cudaStream_t st = b->stream;

@@ -2,13 +2,13 @@
 // grid of at most one block per SM with a barrier in global memory.
 #include <stdint.h>
 
-#include <algorithm>
-
 #include "fa2_build.cuh"
 
 namespace fa2 {
 
 namespace {
+
+constexpr int kBuildThreads = 512;
 
 // The blocks of one cooperative launch (all of them resident).  The barrier
 // counts arrivals in a word that is zero when the launch starts.  A wait that
@@ -52,8 +52,8 @@ struct GridTeam {
 // share the SMs with it.
 __global__ void __launch_bounds__(kBuildThreads, 2) k_build(BuildArgs A, int chunk,
                                                             DevState *st, IterCounters *ctr) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    BuildSmem &S = *reinterpret_cast<BuildSmem *>(smem_raw);
+    extern __shared__ __align__(64) unsigned char smem_raw[];
+    BuildSmem<kBuildThreads> &S = *reinterpret_cast<BuildSmem<kBuildThreads> *>(smem_raw);
     if (st->err || st->poison) return;
     A.rootx = st->rootx;
     A.rooty = st->rooty;
@@ -110,10 +110,9 @@ void launch_build(const Buffers &b, bool keep_moments, int nsm, cudaStream_t s) 
     attr[0].val.cooperative = 1;
     cudaLaunchConfig_t cfg{};
     const int blocks = build_blocks(b.n, nsm);
-    // a tile in one chunk where it fits
-    const int chunk = std::min(kBuildChunk, std::max(kBuildThreads, build_tile(b.n, blocks)));
+    const int chunk = build_chunk(build_tile(b.n, blocks), kBuildThreads);
     cfg.gridDim = dim3((unsigned)blocks);
-    cfg.dynamicSmemBytes = build_smem_bytes(chunk);
+    cfg.dynamicSmemBytes = build_smem_bytes<kBuildThreads>(chunk);
     cfg.blockDim = dim3(kBuildThreads);
     cfg.stream = s;
     cfg.attrs = attr;
@@ -123,7 +122,7 @@ void launch_build(const Buffers &b, bool keep_moments, int nsm, cudaStream_t s) 
 
 void build_set_smem_attr() {
     cudaFuncSetAttribute(k_build, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)build_smem_bytes(kBuildChunk));
+                         (int)build_smem_bytes<kBuildThreads>(kBuildThreads * kBuildRounds));
 }
 
 size_t build_totals_bytes(int blocks) { return (size_t)blocks * sizeof(NodeSums); }

@@ -50,10 +50,7 @@
 
 namespace fa2 {
 
-constexpr int kBuildThreads = 512;
-constexpr int kBuildWarps = kBuildThreads / kWarp;
-constexpr int kBuildRounds = 9;                            // keys per thread in a sort chunk
-constexpr int kBuildChunk = kBuildThreads * kBuildRounds;  // at most, 4608 keys
+constexpr int kBuildRounds = 9;  // keys per thread in a sort chunk, at most
 constexpr int kCellLevels = 5;  // levels whose largest cell is tracked: 12, 16, 20, 24, 28
 
 struct NodeSums {
@@ -143,22 +140,25 @@ __host__ __device__ inline int build_tile(int n, int size) {
 
 constexpr int kMinRows = 256;
 
+// T: threads per block (256 or 512).
+template <int T>
 struct BuildSmem {
+    static constexpr int kThreads = T, kWarps = T / kWarp;
     union {
-        uint32_t whist[kBuildWarps][256];  // per-warp digit counts, then offsets
+        uint32_t whist[kWarps][256];  // per-warp digit counts, then offsets
         struct {
-            uint4 before[8][64], all[8][64];  // partial sums over the count rows
+            uint4 before[T / 64][64], all[T / 64][64];  // partial sums over the count rows
         } rows;
         struct {
-            NodeSums warp[kBuildWarps];
+            NodeSums warp[kWarps];
             NodeSums prefix;
-            uint32_t least[kBuildWarps];
-            int deepest[kBuildWarps];
+            uint32_t least[kWarps];
+            int deepest[kWarps];
         } scan;
     };
     uint32_t base[256];      // next output position of each digit
     uint32_t tile_off[256];  // exclusive scan of the chunk's digit counts
-    uint32_t qsum[2][256];
+    uint32_t qsum[T / 256][256];
     uint32_t scan_w[8];
     int cells[kCellLevels + 3];
     // the tile's least shared digits per row (up to kMinRows rows), and every
@@ -170,13 +170,20 @@ struct BuildSmem {
         return reinterpret_cast<uint64_t *>(this + 1);
     }
 };
-__host__ __device__ inline size_t build_smem_bytes(int chunk) {
-    return sizeof(BuildSmem) + (size_t)chunk * 12;
+// Keys a tile's sort stages at a time: the tile where it fits.
+inline int build_chunk(int tile, int threads) {
+    const int most = threads * kBuildRounds;
+    return tile > most ? most : (tile < threads ? threads : tile);
+}
+template <int T>
+size_t build_smem_bytes(int chunk) {
+    return sizeof(BuildSmem<T>) + (size_t)chunk * 12;
 }
 
 // Exclusive scan of v over threads 0..255 (every thread of the block calls;
 // the others' results are unused).
-__device__ __forceinline__ uint32_t scan256(uint32_t v, BuildSmem &S) {
+template <int T>
+__device__ __forceinline__ uint32_t scan256(uint32_t v, BuildSmem<T> &S) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t inc = v;
 #pragma unroll
@@ -194,166 +201,21 @@ __device__ __forceinline__ uint32_t scan256(uint32_t v, BuildSmem &S) {
     return b + inc - v;
 }
 
-// One stable pass over this block's tile [t0, t1): digit `pass` from kin/vin
-// to kout/vout.  counts rows of `pass` are complete; the next pass's rows get
-// the counts of its digits per output tile.
-template <class Team>
-__device__ __forceinline__ void build_pass(const BuildArgs &A, const Team &team, int pass,
-                                           const uint64_t *kin, const uint32_t *vin,
-                                           uint64_t *kout, uint32_t *vout, int t0, int t1,
-                                           int tile, int chunk, BuildSmem &S) {
-    uint64_t *stage_k = S.stage_keys();
-    uint32_t *stage_v = reinterpret_cast<uint32_t *>(stage_k + chunk);
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int shift = 8 * pass;
-    const unsigned lt = (1u << lane) - 1u;
-    // the digits' starts: keys of smaller digits anywhere, and of this digit
-    // in the tiles before
-    {
-        const uint4 *row = reinterpret_cast<const uint4 *>(A.counts) +
-                           (size_t)pass * team.size * 64 + (tid & 63);
-        uint4 before = make_uint4(0, 0, 0, 0), all = before;
-#pragma unroll 4
-        for (int t = tid >> 6; t < team.size; t += kBuildThreads / 64) {
-            const uint4 c = __ldcg(row + (size_t)t * 64);
-            all.x += c.x;
-            all.y += c.y;
-            all.z += c.z;
-            all.w += c.w;
-            if (t < team.rank) {
-                before.x += c.x;
-                before.y += c.y;
-                before.z += c.z;
-                before.w += c.w;
-            }
-        }
-        S.rows.before[tid >> 6][tid & 63] = before;
-        S.rows.all[tid >> 6][tid & 63] = all;
-        __syncthreads();
-        uint32_t b = 0, a = 0;
-        if (tid < 256) {
-#pragma unroll
-            for (int g = 0; g < kBuildThreads / 64; ++g) {
-                b += reinterpret_cast<const uint32_t *>(S.rows.before[g])[tid];
-                a += reinterpret_cast<const uint32_t *>(S.rows.all[g])[tid];
-            }
-        }
-        const uint32_t ex = scan256(a, S);
-        if (tid < 256) S.base[tid] = ex + b;
-    }
-    uint32_t *next = pass < 7 ? A.counts + (size_t)(pass + 1) * team.size * 256 : nullptr;
-    for (int c0 = t0; c0 < t1; c0 += chunk) {
-        const int cn = min(chunk, t1 - c0);
-        const int rounds = (cn + kBuildThreads - 1) / kBuildThreads;
-        const int w0 = c0 + wid * rounds * 32;
-        uint64_t k[kBuildRounds];
-        uint32_t v[kBuildRounds], rank[kBuildRounds];
-#pragma unroll
-        for (int r = 0; r < kBuildRounds; ++r) {
-            const int i = w0 + r * 32 + lane;
-            const bool in = r < rounds && i < t1;
-            k[r] = in ? kin[i] : 0ull;
-            v[r] = in ? vin[i] : 0u;
-        }
-        for (int j = tid; j < kBuildWarps * 256; j += kBuildThreads) (&S.whist[0][0])[j] = 0;
-        __syncthreads();
-        // rank by digit per warp, in key order: the lanes that share a digit
-        // are the AND of eight ballots
-#pragma unroll
-        for (int r = 0; r < kBuildRounds; ++r) {
-            if (r < rounds) {
-                const bool valid = w0 + r * 32 + lane < t1;
-                const uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
-                unsigned peers = __ballot_sync(kFullMask, valid);
-                if (!valid) peers = ~peers;
-#pragma unroll
-                for (int b = 0; b < 8; ++b) {
-                    const bool bit = (d >> b) & 1u;
-                    const unsigned m = __ballot_sync(kFullMask, bit);
-                    peers &= bit ? m : ~m;
-                }
-                uint32_t before = 0;
-                if (valid) before = S.whist[wid][d];
-                rank[r] = before + __popc(peers & lt);
-                __syncwarp();
-                if (valid && (peers & lt) == 0) S.whist[wid][d] = before + __popc(peers);
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        // per digit: offsets across the warps, two threads per digit
-        const int dg = tid & 255, half = tid >> 8;
-        uint32_t q = 0;
-#pragma unroll
-        for (int w = 0; w < kBuildWarps / 2; ++w) q += S.whist[half * (kBuildWarps / 2) + w][dg];
-        S.qsum[half][dg] = q;
-        __syncthreads();
-        uint32_t run = half ? S.qsum[0][dg] : 0u;
-        const uint32_t total = S.qsum[0][dg] + S.qsum[1][dg];
-#pragma unroll
-        for (int w = 0; w < kBuildWarps / 2; ++w) {
-            const uint32_t c = S.whist[half * (kBuildWarps / 2) + w][dg];
-            S.whist[half * (kBuildWarps / 2) + w][dg] = run;
-            run += c;
-        }
-        const uint32_t ex = scan256(total, S);
-        if (half == 0) S.tile_off[dg] = ex;
-        __syncthreads();
-        // regroup by digit in shared memory, write digit runs, count the next
-        // pass's digits per output tile
-#pragma unroll
-        for (int r = 0; r < kBuildRounds; ++r) {
-            if (r < rounds && w0 + r * 32 + lane < t1) {
-                const uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
-                const uint32_t p = S.tile_off[d] + S.whist[wid][d] + rank[r];
-                stage_k[p] = k[r];
-                stage_v[p] = v[r];
-            }
-        }
-        __syncthreads();
-        for (int j = tid; j < cn; j += kBuildThreads) {
-            const uint64_t key = stage_k[j];
-            const uint32_t d = (uint32_t)(key >> shift) & 255u;
-            const uint32_t out = S.base[d] + (uint32_t)j - S.tile_off[d];
-            kout[out] = key;
-            vout[out] = stage_v[j];
-            if (next)
-                atomicAdd(&next[(size_t)(out / (uint32_t)tile) * 256 +
-                                ((uint32_t)(key >> (shift + 8)) & 255u)],
-                          1u);
-        }
-        __syncthreads();
-        if (half == 0) S.base[dg] += total;
-        __syncthreads();
-    }
-}
-
-// This block's row of the counts of digit `first` from `keys`, and zeros in
-// its rows of the later passes.
-template <class Team>
-__device__ __forceinline__ void build_count_rows(const BuildArgs &A, const Team &team, int first,
-                                                 BuildSmem &S) {
-    for (int j = threadIdx.x; j < (8 - first) * 256; j += kBuildThreads) {
-        const int p = first + (j >> 8);
-        A.counts[((size_t)p * team.size + team.rank) * 256 + (j & 255)] =
-            p == first ? S.base[j & 255] : 0u;
-    }
-}
-
 // The fix phase of this block's tile: every key of a run of keys equal above
 // `low` bits goes to its place by (key, input position), the others keep
 // theirs.
+template <int T>
 __device__ __forceinline__ void build_fix(const BuildArgs &A, int low, const uint64_t *kin,
                                           const uint32_t *vin, uint64_t *kout, uint32_t *vout,
                                           int t0, int t1) {
     const int n = A.n;
-    for (int i = t0 + (int)threadIdx.x; i < t1; i += kBuildThreads) {
+    for (int i = t0 + (int)threadIdx.x; i < t1; i += T) {
         const uint64_t key = kin[i];
         const uint32_t v = vin[i];
         const uint64_t hk = key >> low;
         int to = i;
-        const bool left = i > 0 && (kin[i - 1] >> low) == hk;
-        const bool right = i + 1 < n && (kin[i + 1] >> low) == hk;
+        const bool left = low > 0 && i > 0 && (kin[i - 1] >> low) == hk;
+        const bool right = low > 0 && i + 1 < n && (kin[i + 1] >> low) == hk;
         if (left || right) {
             int s = i, smaller = 0;
             while (s > 0 && i - s <= kMaxRun) {
@@ -376,6 +238,228 @@ __device__ __forceinline__ void build_fix(const BuildArgs &A, int low, const uin
         }
         kout[to] = key;
         vout[to] = v;
+    }
+}
+
+// Where each of a chunk's keys goes by the digit at `shift`, stably: at[r] for
+// the thread's key k[r], the (w0 + 32 r + lane)-th, valid below `end`.  Warps
+// hold consecutive keys.  Leaves the digits' first places in S.tile_off and
+// returns the count of digit threadIdx.x & 255.
+template <int T>
+__device__ __forceinline__ uint32_t chunk_order(const uint64_t (&k)[kBuildRounds], int rounds,
+                                                int w0, int end, int shift,
+                                                uint32_t (&at)[kBuildRounds], BuildSmem<T> &S) {
+    constexpr int kWarps = T / kWarp, kQ = T / 256;  // threads per digit
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    for (int j = tid; j < kWarps * 256; j += T) (&S.whist[0][0])[j] = 0;
+    __syncthreads();
+    // rank by digit per warp, in key order: the lanes that share a digit are
+    // the AND of eight ballots
+#pragma unroll
+    for (int r = 0; r < kBuildRounds; ++r) {
+        if (r < rounds) {
+            const bool valid = w0 + r * 32 + lane < end;
+            const uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
+            unsigned peers = __ballot_sync(kFullMask, valid);
+            if (!valid) peers = ~peers;
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const bool bit = (d >> b) & 1u;
+                const unsigned m = __ballot_sync(kFullMask, bit);
+                peers &= bit ? m : ~m;
+            }
+            uint32_t before = 0;
+            if (valid) before = S.whist[wid][d];
+            at[r] = before + __popc(peers & lt);
+            __syncwarp();
+            if (valid && (peers & lt) == 0) S.whist[wid][d] = before + __popc(peers);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    // per digit: offsets across the warps, eight warps per thread
+    const int dg = tid & 255, part = tid >> 8;
+    uint32_t q = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps / kQ; ++w) q += S.whist[part * (kWarps / kQ) + w][dg];
+    S.qsum[part][dg] = q;
+    __syncthreads();
+    uint32_t run = 0, total = 0;
+#pragma unroll
+    for (int h = 0; h < kQ; ++h) {
+        const uint32_t c = S.qsum[h][dg];
+        if (h < part) run += c;
+        total += c;
+    }
+#pragma unroll
+    for (int w = 0; w < kWarps / kQ; ++w) {
+        const uint32_t c = S.whist[part * (kWarps / kQ) + w][dg];
+        S.whist[part * (kWarps / kQ) + w][dg] = run;
+        run += c;
+    }
+    const uint32_t ex = scan256(total, S);
+    if (part == 0) S.tile_off[dg] = ex;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kBuildRounds; ++r) {
+        if (r < rounds && w0 + r * 32 + lane < end) {
+            const uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
+            at[r] += S.tile_off[d] + S.whist[wid][d];
+        }
+    }
+    return total;
+}
+
+// One stable pass over this block's tile [t0, t1): digit `pass` from kin/vin
+// to kout/vout.  counts rows of `pass` are complete; the next pass's rows get
+// the counts of its digits per output tile.
+template <int T, class Team>
+__device__ __forceinline__ void build_pass(const BuildArgs &A, const Team &team, int pass,
+                                           const uint64_t *kin, const uint32_t *vin,
+                                           uint64_t *kout, uint32_t *vout, int t0, int t1,
+                                           int tile, int chunk, BuildSmem<T> &S) {
+    uint64_t *stage_k = S.stage_keys();
+    uint32_t *stage_v = reinterpret_cast<uint32_t *>(stage_k + chunk);
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int shift = 8 * pass;
+    // the digits' starts: keys of smaller digits anywhere, and of this digit
+    // in the tiles before
+    {
+        const uint4 *row = reinterpret_cast<const uint4 *>(A.counts) +
+                           (size_t)pass * team.size * 64 + (tid & 63);
+        uint4 before = make_uint4(0, 0, 0, 0), all = before;
+#pragma unroll 4
+        for (int t = tid >> 6; t < team.size; t += T / 64) {
+            const uint4 c = __ldcg(row + (size_t)t * 64);
+            all.x += c.x;
+            all.y += c.y;
+            all.z += c.z;
+            all.w += c.w;
+            if (t < team.rank) {
+                before.x += c.x;
+                before.y += c.y;
+                before.z += c.z;
+                before.w += c.w;
+            }
+        }
+        S.rows.before[tid >> 6][tid & 63] = before;
+        S.rows.all[tid >> 6][tid & 63] = all;
+        __syncthreads();
+        uint32_t b = 0, a = 0;
+        if (tid < 256) {
+#pragma unroll
+            for (int g = 0; g < T / 64; ++g) {
+                b += reinterpret_cast<const uint32_t *>(S.rows.before[g])[tid];
+                a += reinterpret_cast<const uint32_t *>(S.rows.all[g])[tid];
+            }
+        }
+        const uint32_t ex = scan256(a, S);
+        if (tid < 256) S.base[tid] = ex + b;
+    }
+    uint32_t *next = pass < 7 ? A.counts + (size_t)(pass + 1) * team.size * 256 : nullptr;
+    for (int c0 = t0; c0 < t1; c0 += chunk) {
+        const int cn = min(chunk, t1 - c0);
+        const int rounds = (cn + T - 1) / T;
+        const int w0 = c0 + wid * rounds * 32;
+        uint64_t k[kBuildRounds];
+        uint32_t v[kBuildRounds], at[kBuildRounds];
+#pragma unroll
+        for (int r = 0; r < kBuildRounds; ++r) {
+            const int i = w0 + r * 32 + lane;
+            const bool in = r < rounds && i < t1;
+            k[r] = in ? kin[i] : 0ull;
+            v[r] = in ? vin[i] : 0u;
+        }
+        const uint32_t total = chunk_order(k, rounds, w0, t1, shift, at, S);
+        // regroup by digit in shared memory, write digit runs, count the next
+        // pass's digits per output tile
+#pragma unroll
+        for (int r = 0; r < kBuildRounds; ++r) {
+            if (r < rounds && w0 + r * 32 + lane < t1) {
+                stage_k[at[r]] = k[r];
+                stage_v[at[r]] = v[r];
+            }
+        }
+        __syncthreads();
+        for (int j = tid; j < cn; j += T) {
+            const uint64_t key = stage_k[j];
+            const uint32_t d = (uint32_t)(key >> shift) & 255u;
+            const uint32_t out = S.base[d] + (uint32_t)j - S.tile_off[d];
+            kout[out] = key;
+            vout[out] = stage_v[j];
+            if (next)
+                atomicAdd(&next[(size_t)(out / (uint32_t)tile) * 256 +
+                                ((uint32_t)(key >> (shift + 8)) & 255u)],
+                          1u);
+        }
+        __syncthreads();
+        if (tid < 256) S.base[tid] += total;
+        __syncthreads();
+    }
+}
+
+// The keys and every pass of a graph that one block's staging holds, in
+// registers and shared memory; the order goes to keys[0], vals[0].
+template <int T>
+__device__ __forceinline__ void build_sort_local(const BuildArgs &A, int first, int chunk,
+                                                 BuildSmem<T> &S) {
+    const int n = A.n, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    uint64_t *stage_k = S.stage_keys();
+    uint32_t *stage_v = reinterpret_cast<uint32_t *>(stage_k + chunk);
+    const int rounds = (n + T - 1) / T, w0 = wid * rounds * 32;
+    uint64_t k[kBuildRounds];
+    uint32_t v[kBuildRounds], at[kBuildRounds];
+#pragma unroll
+    for (int r = 0; r < kBuildRounds; ++r) {
+        const int i = w0 + r * 32 + lane;
+        k[r] = 0ull;
+        v[r] = (uint32_t)i;
+        if (r < rounds && i < n) {
+            const float2 p = A.pos[i];
+            k[r] = morton_key(p.x, p.y, A.rootx, A.rooty, A.radius);
+        }
+    }
+    for (;;) {
+        for (int pass = first; pass < 8; ++pass) {
+            chunk_order(k, rounds, w0, n, 8 * pass, at, S);
+#pragma unroll
+            for (int r = 0; r < kBuildRounds; ++r) {
+                if (r < rounds && w0 + r * 32 + lane < n) {
+                    stage_k[at[r]] = k[r];
+                    stage_v[at[r]] = v[r];
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < kBuildRounds; ++r) {
+                const int i = w0 + r * 32 + lane;
+                if (r < rounds && i < n) {
+                    k[r] = stage_k[i];
+                    v[r] = stage_v[i];
+                }
+            }
+            __syncthreads();
+        }
+        // with every digit sorted there is nothing to put in order
+        build_fix<T>(A, 8 * first, stage_k, stage_v, A.keys[0], A.vals[0], 0, n);
+        __syncthreads();
+        if (first == 0 || !*(volatile int *)A.resort) break;
+        // a run too long: every digit, from the order the partial sort left
+        if (tid == 0) *A.resorts += 1;
+        first = 0;
+    }
+}
+
+// This block's row of the counts of digit `first` from `keys`, and zeros in
+// its rows of the later passes.
+template <int T, class Team>
+__device__ __forceinline__ void build_count_rows(const BuildArgs &A, const Team &team, int first,
+                                                 BuildSmem<T> &S) {
+    for (int j = threadIdx.x; j < (8 - first) * 256; j += T) {
+        const int p = first + (j >> 8);
+        A.counts[((size_t)p * team.size + team.rank) * 256 + (j & 255)] =
+            p == first ? S.base[j & 255] : 0u;
     }
 }
 
@@ -463,8 +547,9 @@ struct CountOut {
     int deepest;     // most shared digits
     uint32_t least;  // least shared digits + 1
 };
+template <int T>
 __device__ __forceinline__ CountOut build_count(const BuildArgs &A, int r0, int r1, int tile_r0,
-                                                double scale, BuildSmem &S) {
+                                                double scale, BuildSmem<T> &S) {
     const int n = A.n, lane = threadIdx.x & 31;
     CountOut out{{0, 0, 0, 0}, 0, 255u};
     constexpr int kB = 3;  // rows whose loads are in flight together
@@ -529,9 +614,10 @@ __device__ __forceinline__ CountOut build_count(const BuildArgs &A, int r0, int 
 // The whole build.  Team: rank, size and sync(), a barrier of its blocks that
 // orders their global memory accesses and returns false when it gave up.
 // `chunk` is the number of keys the shared memory stages.
-template <class Team>
-__device__ __forceinline__ void build_tree(const BuildArgs &A, Team &team, BuildSmem &S,
+template <int T, class Team>
+__device__ __forceinline__ void build_tree(const BuildArgs &A, Team &team, BuildSmem<T> &S,
                                            int chunk) {
+    constexpr int kWarps = T / kWarp;
     const int n = A.n, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int tile = build_tile(n, team.size);
     const int t0 = min(n, team.rank * tile), t1 = min(n, t0 + tile);
@@ -544,53 +630,60 @@ __device__ __forceinline__ void build_tree(const BuildArgs &A, Team &team, Build
         *A.resort = 0;
         *A.deep = 0;
     }
-    // ---- keys
-    if (tid < 256) S.base[tid] = 0;
     if (tid < kCellLevels) S.cells[tid] = 0;
-    __syncthreads();
-    for (int i = t0 + tid; i < t1; i += kBuildThreads) {
-        const float2 p = A.pos[i];
-        const uint64_t key = morton_key(p.x, p.y, A.rootx, A.rooty, A.radius);
-        K(cur)[i] = key;
-        V(cur)[i] = (uint32_t)i;
-        atomicAdd(&S.base[(uint32_t)(key >> (8 * first)) & 255u], 1u);
-    }
-    __syncthreads();
-    build_count_rows(A, team, first, S);
-    if (!team.sync()) return;
-    // every block has read the plan
-    if (team.rank == 0 && tid < kCellLevels) A.cells[tid] = 0;
-    // ---- sort
-    for (int pass = first; pass < 8; ++pass, cur ^= 1) {
-        build_pass(A, team, pass, K(cur), V(cur), K(cur ^ 1), V(cur ^ 1), t0, t1, tile, chunk, S);
+    if (team.size == 1 && n <= chunk) {
+        // ---- keys and sort within the block
+        __syncthreads();  // every thread has read the plan
+        if (tid < kCellLevels) A.cells[tid] = 0;
+        build_sort_local(A, first, chunk, S);
+    } else {
+        // ---- keys
+        if (tid < 256) S.base[tid] = 0;
+        __syncthreads();
+        for (int i = t0 + tid; i < t1; i += T) {
+            const float2 p = A.pos[i];
+            const uint64_t key = morton_key(p.x, p.y, A.rootx, A.rooty, A.radius);
+            K(cur)[i] = key;
+            V(cur)[i] = (uint32_t)i;
+            atomicAdd(&S.base[(uint32_t)(key >> (8 * first)) & 255u], 1u);
+        }
+        __syncthreads();
+        build_count_rows(A, team, first, S);
         if (!team.sync()) return;
-    }
-    if (first > 0) {
-        build_fix(A, 8 * first, K(cur), V(cur), K(cur ^ 1), V(cur ^ 1), t0, t1);
-        cur ^= 1;
-        if (!team.sync()) return;
-        if (*(volatile int *)A.resort) {
-            if (team.rank == 0 && tid == 0) *A.resorts += 1;
-            // every digit, from the order the partial sort left: equal keys
-            // keep their input order through both, so this is the full
-            // sort's order
-            if (tid < 256) S.base[tid] = 0;
-            __syncthreads();
-            for (int i = t0 + tid; i < t1; i += kBuildThreads)
-                atomicAdd(&S.base[(uint32_t)K(cur)[i] & 255u], 1u);
-            __syncthreads();
-            build_count_rows(A, team, 0, S);
+        // every block has read the plan
+        if (team.rank == 0 && tid < kCellLevels) A.cells[tid] = 0;
+        // ---- sort
+        for (int pass = first; pass < 8; ++pass, cur ^= 1) {
+            build_pass(A, team, pass, K(cur), V(cur), K(cur ^ 1), V(cur ^ 1), t0, t1, tile, chunk, S);
             if (!team.sync()) return;
-            for (int pass = 0; pass < 8; ++pass, cur ^= 1) {
-                build_pass(A, team, pass, K(cur), V(cur), K(cur ^ 1), V(cur ^ 1), t0, t1, tile,
-                           chunk, S);
+        }
+        if (first > 0) {
+            build_fix<T>(A, 8 * first, K(cur), V(cur), K(cur ^ 1), V(cur ^ 1), t0, t1);
+            cur ^= 1;
+            if (!team.sync()) return;
+            if (*(volatile int *)A.resort) {
+                if (team.rank == 0 && tid == 0) *A.resorts += 1;
+                // every digit, from the order the partial sort left: equal keys
+                // keep their input order through both, so this is the full
+                // sort's order
+                if (tid < 256) S.base[tid] = 0;
+                __syncthreads();
+                for (int i = t0 + tid; i < t1; i += T)
+                    atomicAdd(&S.base[(uint32_t)K(cur)[i] & 255u], 1u);
+                __syncthreads();
+                build_count_rows(A, team, 0, S);
                 if (!team.sync()) return;
+                for (int pass = 0; pass < 8; ++pass, cur ^= 1) {
+                    build_pass(A, team, pass, K(cur), V(cur), K(cur ^ 1), V(cur ^ 1), t0, t1, tile,
+                               chunk, S);
+                    if (!team.sync()) return;
+                }
             }
         }
     }
     // ---- count: the warps' and tiles' sums
     const double scale = A.radius > 0.0f ? kFixedScale / (double)A.radius : 1.0;
-    const int rows = (t1 - t0 + 31) >> 5, per = (rows + kBuildWarps - 1) / kBuildWarps;
+    const int rows = (t1 - t0 + 31) >> 5, per = (rows + kWarps - 1) / kWarps;
     const int r0 = (t0 >> 5) + min(rows, wid * per), r1 = (t0 >> 5) + min(rows, (wid + 1) * per);
     for (bool fixed = false;; fixed = true) {
         const CountOut c = build_count(A, r0, r1, t0 >> 5, scale, S);
@@ -603,23 +696,23 @@ __device__ __forceinline__ void build_tree(const BuildArgs &A, Team &team, Build
         if (wid == 0) {
             // the warps' exclusive sums, and the tile's
             const NodeSums zero{0, 0, 0, 0};
-            const NodeSums w = lane < kBuildWarps ? S.scan.warp[lane] : zero;
+            const NodeSums w = lane < kWarps ? S.scan.warp[lane] : zero;
             NodeSums wi = w;
 #pragma unroll
-            for (int o = 1; o < kBuildWarps; o <<= 1) {
+            for (int o = 1; o < kWarps; o <<= 1) {
                 const NodeSums t = shfl_up_sums(wi, o);
                 if (lane >= o) sums_add(wi, t);
             }
-            if (lane == kBuildWarps - 1) A.totals[team.rank] = wi;
+            if (lane == kWarps - 1) A.totals[team.rank] = wi;
             wi.g -= w.g;
             wi.m -= w.m;
             wi.x -= w.x;
             wi.y -= w.y;
-            if (lane < kBuildWarps) S.scan.warp[lane] = wi;
+            if (lane < kWarps) S.scan.warp[lane] = wi;
             const uint32_t least =
-                __reduce_min_sync(kFullMask, lane < kBuildWarps ? S.scan.least[lane] : 255u);
+                __reduce_min_sync(kFullMask, lane < kWarps ? S.scan.least[lane] : 255u);
             const int deepest =
-                __reduce_max_sync(kFullMask, lane < kBuildWarps ? S.scan.deepest[lane] : 0);
+                __reduce_max_sync(kFullMask, lane < kWarps ? S.scan.deepest[lane] : 0);
             if (lane == 0) {
                 A.tilemin[team.rank] = (uint8_t)least;
                 atomicMax(A.max_level, deepest);
@@ -630,7 +723,7 @@ __device__ __forceinline__ void build_tree(const BuildArgs &A, Team &team, Build
         if (fixed || !*(volatile int *)A.deep) break;
         // runs of equal 64-bit keys: in the order of the digits below, then
         // the count again
-        for (int k = t0 + tid; k < t1; k += kBuildThreads)
+        for (int k = t0 + tid; k < t1; k += T)
             if (A.lcp[k] == kLevels + 1 && (k == 0 || A.lcp[k - 1] != kLevels + 1))
                 fix_run(k, n, A.keys[0], A.vals[0], A.pos, A.ref_of, A.rootx, A.rooty, A.radius,
                         A.err, A.poison, 0);

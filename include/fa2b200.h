@@ -405,11 +405,12 @@ int fa2_batch_step_timed(fa2_batch *batch, int32_t n_iters, float *ms);
  * per node, same order as the positions); the body order of each graph's
  * quadtree (graph-local ids, the reference's sortd); the adaptive speed and
  * speed efficiency per graph. */
-/* CTA sizes: graphs of at most `split` nodes run on CTAs of small_threads
- * threads beside the others on CTAs of large_threads threads (each 256, 512
- * or 1024), each class from its own queue; the default is split 0 with
- * 1024-thread CTAs, one class.  Results do not depend on the choice, only the
- * speed does. */
+/* CTA sizes: graphs of at most `split` nodes run with small_threads beside the
+ * others with large_threads (each 256, 512 or 1024): 256 is one CTA of 256
+ * threads per graph; 512 and 1024 are CTAs of 512 threads, one for a small
+ * graph and a cluster of up to eight for a large one.  Each size class has its
+ * own queue; the default is split 0 with 1024.  Results do not depend on the
+ * choice, only the speed does. */
 int fa2_batch_configure(fa2_batch *batch, uint32_t split, int32_t small_threads,
                         int32_t large_threads);
 int fa2_batch_get_config(fa2_batch *batch, uint32_t *split, int32_t *small_threads,
