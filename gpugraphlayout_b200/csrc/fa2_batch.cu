@@ -66,7 +66,7 @@ struct BatchCtl {
 // Offsets of one team's scratch slot, in bytes, each 256-byte aligned.
 struct SlotLayout {
     size_t ctl, keys0, keys1, vals0, vals1, sbody, lcp, rowmin, tilemin, defer, group, body_node,
-        owner, nodes, pm, pxy, counts, totals, fa, f, gpart;
+        owner, nodes, pm, pxy, counts, hist, totals, fa, f, gpart;
     size_t bytes;
     uint32_t cap;  // tree nodes a slot holds
 };
@@ -389,7 +389,9 @@ __global__ void __launch_bounds__(T, kBatchThreadsPerSm / T) k_batch(BatchArgs A
         T_.pm = slot_ptr<long long>(slot, A.L.pm);
         T_.pxy = slot_ptr<i128>(slot, A.L.pxy);
         T_.counts = slot_ptr<uint32_t>(slot, A.L.counts);
+        T_.hist = slot_ptr<uint32_t>(slot, A.L.hist);
         T_.totals = slot_ptr<NodeSums>(slot, A.L.totals);
+        for (int j = tid0; j < kBuildBins; j += stride) T_.hist[j] = 0;
         T_.err = &ctl->err;
         T_.poison = &ctl->poison;
         T_.resort = &ctl->resort;
@@ -488,6 +490,7 @@ SlotLayout make_layout(uint32_t nmax, int team) {
     L.pm = take(8ull * (nmax + 1));
     L.pxy = take(32ull * (nmax + 1));
     L.counts = take(4ull * build_counts(team));
+    L.hist = take(4ull * kBuildBins);
     L.totals = take(build_totals_bytes(team));
     L.fa = take(8ull * nmax);
     L.f = take(8ull * nmax);

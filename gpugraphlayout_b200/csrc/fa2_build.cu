@@ -9,6 +9,7 @@ namespace fa2 {
 namespace {
 
 constexpr int kBuildThreads = 512;
+static_assert(kBuildThreads * kBinsPerThread == kBuildBins, "the bins' counts");
 
 // The blocks of one cooperative launch (all of them resident).  The barrier
 // counts arrivals in a word that is zero when the launch starts.  A wait that
@@ -96,6 +97,7 @@ void launch_build(const Buffers &b, bool keep_moments, int nsm, cudaStream_t s) 
     A.mom_q = keep_moments ? b.mom_q : nullptr;
     A.mom_m = keep_moments ? b.mom_m : nullptr;
     A.counts = b.sort_counts;
+    A.hist = b.ctr->hist;
     A.totals = static_cast<NodeSums *>(b.build_totals);
     A.err = &b.st->err;
     A.poison = &b.st->poison;

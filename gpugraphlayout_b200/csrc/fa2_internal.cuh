@@ -48,10 +48,13 @@ struct DevState {
     float trav_radius;                // root radius the last traversal used
     int resort;                       // this sort skipped low digits that it needs
     int deep;                         // bodies that share a whole 64-bit key
-    int cells[5];                     // largest cell of the last tree at levels 12, 16, .., 28
+    int cells[6];                     // largest cell of the last tree at levels 12, 16, .., 28, 6
 };
 
-// Per-iteration scratch, cleared by one memset at the start of an iteration.
+constexpr int kBuildBins = 4096;
+
+// Counters at zero between iterations: each is cleared by the kernels that are
+// done with it.
 struct IterCounters {
     unsigned bbox_done;
     unsigned build_bar;  // barrier arrivals of the tree build
@@ -61,6 +64,7 @@ struct IterCounters {
     unsigned mom_ticket;
     unsigned pad[2];
     unsigned pair_count[16];  // (group, cell) pairs of a learned walk, per pair segment
+    unsigned hist[kBuildBins];  // keys per bin of the tree build's bucket sort
 };
 
 // Blocks of the tree build: 512 bodies or more each, at most one per SM.

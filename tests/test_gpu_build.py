@@ -1,0 +1,128 @@
+"""The tree build at the sizes and crowdings where its paths change.
+
+One block sorts in shared memory up to 512 bodies; more blocks by buckets up
+to 1024 bodies each, and beyond that, or where more than 128 bodies share one
+of the buckets' squares, by radix passes with a fix-up.  The choice looks at
+the tree before, so each layout is built first after a fresh start and again
+after another one.  The body order is the oracle's exactly on every path; the
+repulsion sums the same terms in another order (float32: under 1e-4 relative
+for sums of up to 1500 terms, the suite's bar).
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_rmse
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-4
+
+
+def _graph(n):
+    from oracle import oracle as O
+    s = np.arange(n, dtype=np.uint32)
+    return O.Graph(s, np.roll(s, -1)) if n > 2 else O.Graph(s[:1], s[1:2])
+
+
+def _uniform(n, seed):
+    """Two bodies at opposite corners pin the root box to [-1024, 1024]^2; the
+    others keep out of the level-6 cell [0, 32)^2."""
+    rng = np.random.default_rng(seed)
+    xy = rng.uniform(-1000, 1000, (n, 2))
+    xy[:, 0] = np.where((xy >= 0).all(1) & (xy < 32).all(1), xy[:, 0] - 500, xy[:, 0])
+    xy[0], xy[1] = (-1024, -1024), (1024, 1024)
+    return xy.astype(np.float32)
+
+
+def _crowd(n, count, seed, kind):
+    """`count` bodies in that cell: spread over it, or in one cell of level 24;
+    "equal": some of them share all 64 bits of their keys."""
+    xy = _uniform(n, seed)
+    rng = np.random.default_rng(seed + 1)
+    w = 30.0 if kind == "spread" else 2048.0 / 2 ** 24
+    side = int(np.ceil(np.sqrt(count)))
+    grid = rng.permutation(side * side)[:count]
+    xy[2:2 + count, 0] = (grid % side + 0.5) * (w / side)
+    xy[2:2 + count, 1] = (grid // side + 0.5) * (w / side)
+    if kind == "equal":
+        xy[2:5] = [(1e-9, 1e-9), (3e-9, 1e-9), (2e-9, 4e-9)]
+    return xy
+
+
+def _check(e, xy, mass, forces):
+    from oracle import oracle as O
+    e.set_positions(xy)
+    e.step(1)
+    st = e.stats()
+    assert st["device_error"] == 0
+    t = O.Tree(xy, mass)
+    assert np.array_equal(e.sort_order(), t.sort().astype(np.uint32))
+    if forces:
+        tot, ga = e.forces()
+        ref, overflow, _ = t.repulsion(10.0)
+        assert overflow or rel_rmse(tot - ga, ref) <= TOL
+
+
+# 1 and 2 blocks; the edges of 148 blocks' tiles of 512 and 1024 bodies
+@pytest.mark.parametrize("n", [2, 31, 33, 511, 512, 513, 1025, 4737, 75776, 75777, 151552, 151553])
+def test_order_at_tile_edges(n):
+    from gpugraphlayout_b200 import Engine
+    g = _graph(n)
+    e = Engine(g.n, g.sources, g.targets, scale=10.0)
+    for seed in (1, 2):
+        _check(e, _uniform(n, seed), g.mass, n <= 5000)
+
+
+@pytest.mark.parametrize("kind", ["spread", "tight", "equal"])
+@pytest.mark.parametrize("n,count", [(500, 127), (500, 128), (500, 129), (500, 400),
+                                     (3000, 128), (3000, 129), (3000, 1500)])
+def test_order_of_crowded_bodies(n, count, kind):
+    from gpugraphlayout_b200 import Engine
+    g = _graph(n)
+    e = Engine(g.n, g.sources, g.targets, scale=10.0)
+    for seed in (1, 3):  # the second build knows that the first one's were crowded
+        _check(e, _crowd(n, count, seed, kind), g.mass, kind == "spread")
+    _check(e, _uniform(n, 5), g.mass, True)
+    _check(e, _crowd(n, count, 7, kind), g.mass, kind == "spread")
+
+
+@pytest.mark.parametrize("threads", [None, 256])
+def test_batch_order_at_team_edges(threads):
+    """The teams' sizes (1, 4 and 8 blocks) and a block's staging; 256 threads:
+    one block per graph, whatever its size."""
+    from gpugraphlayout_b200 import BatchEngine
+    from oracle import oracle as O
+    sizes = [2, 512, 513, 2048, 2049, 2304, 2305, 8192, 8193]
+    graphs = [_graph(n) for n in sizes]
+    b = BatchEngine([(g.n, g.sources, g.targets) for g in graphs], scale=10.0)
+    if threads:
+        b.configure(0, threads, threads)
+    for seed in (1, 2):
+        xys = [_crowd(n, n // 8, seed, "spread") if i % 3 == 2 else _uniform(n, seed)
+               for i, n in enumerate(sizes)]
+        b.set_positions(np.concatenate(xys))
+        b.step(1)
+        order = b.sort_order()
+        tot, ga = b.forces()
+        for i, (g, xy) in enumerate(zip(graphs, xys)):
+            t = O.Tree(xy, g.mass)
+            assert np.array_equal(b.part(order, i), t.sort().astype(np.uint32)), i
+            ref, overflow, _ = t.repulsion(10.0)
+            assert overflow or rel_rmse(b.part(tot - ga, i), ref) <= TOL, i
+
+
+@pytest.mark.parametrize("n", [300, 3000])
+def test_one_call_of_many_iterations_equals_one_call_per_iteration(n):
+    """Calls replay four iterations at a time and the rest one by one: the
+    same arithmetic bit for bit."""
+    from gpugraphlayout_b200 import Engine
+    g = _graph(n)
+    out = []
+    for calls in ([9], [1] * 9, [3, 6]):
+        e = Engine(g.n, g.sources, g.targets, scale=10.0)
+        e.set_positions(_uniform(n, 4))
+        for k in calls:
+            e.step(k)
+        out.append(e.get_positions())
+    assert np.array_equal(out[0], out[1])
+    assert np.array_equal(out[0], out[2])
