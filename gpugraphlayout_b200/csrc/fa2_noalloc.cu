@@ -74,10 +74,11 @@ constexpr int kErrMass = 1 << 8;
 
 // Reference ids (the caller's indices) and the mass check.
 __global__ void k_prepare(uint32_t n, const float *__restrict mass, uint32_t *__restrict ids,
-                          DevState *st) {
+                          float2 *__restrict fag, DevState *st) {
     bool bad = false;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         ids[i] = i;
+        fag[i] = make_float2(0.0f, 0.0f);
         const float m = mass[i];
         bad |= !(m >= 0.0f && m < 16777216.0f && m == truncf(m));
     }
@@ -169,19 +170,17 @@ int run(const float *d_xy, const float *d_mass, uint32_t n, const fa2_params *pr
 
     // Must start at zero on every call: the counters; the device scalars
     // (error and coincidence flags, interaction count; no last tree's cells, so
-    // the sort starts at its shortest); the gravity + attraction term
-    // the traversal adds to the repulsion (zero here, so d_force receives the
-    // repulsion alone).  The reference ids are the caller's indices.
-    cudaError_t e = cudaMemsetAsync(b.ctr, 0, kZeroBytes, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.st, 0, sizeof(DevState), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.fag, 0, (size_t)n * sizeof(float2), s);
+    // the sort takes its shortest way); and the gravity + attraction term the
+    // traversal adds to the repulsion (k_prepare clears it, so d_force receives
+    // the repulsion alone).  The reference ids are the caller's indices.
+    cudaError_t e = cudaMemsetAsync(b.ctr, 0, kOffSt + sizeof(DevState), s);
     if (e != cudaSuccess) return status_of(e);
     // A launch error is read from the runtime's last-error slot.  An error
     // the caller left there before this call is not ours to report or to
     // clear, so launch errors are taken from the slot only if it was empty on
     // entry (otherwise a failed launch still shows in the stream wait below).
     const bool slot_was_clear = cudaPeekAtLastError() == cudaSuccess;
-    k_prepare<<<(n + 255) / 256, 256, 0, s>>>(n, d_mass, const_cast<uint32_t *>(b.ref_of), b.st);
+    k_prepare<<<(n + 255) / 256, 256, 0, s>>>(n, d_mass, const_cast<uint32_t *>(b.ref_of), b.fag, b.st);
     launch_bbox(b, d.nsm * 2, s);
     launch_build(b, false, d.nsm, s);
     launch_traverse(b, kp, d.trav_blocks, s);
