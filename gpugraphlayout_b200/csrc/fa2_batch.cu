@@ -244,10 +244,10 @@ __device__ void phase_traverse(const BatchArgs &A, const ClusterTeam &team, uint
         auto none = [](bool, const float4 &, float, uint32_t) {};
         const float2 a =
             A.prm.epssq >= FLT_MIN
-                ? walk_group<false, false, false, true>(walk[wid], S.dq, nodes, nullptr, nullptr,
+                ? walk_group<false, false, false, true, false>(walk[wid], S.dq, nodes, nullptr, nullptr,
                                                         nullptr, end, px, py, 0.0f, A.prm.epssq,
                                                         none)
-                : walk_group<false, false, false, false>(walk[wid], S.dq, nodes, nullptr, nullptr,
+                : walk_group<false, false, false, false, false>(walk[wid], S.dq, nodes, nullptr, nullptr,
                                                          nullptr, end, px, py, 0.0f, A.prm.epssq,
                                                          none);
         const float kmi = A.prm.k_r * me.z;

@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "fa2_device.cuh"
 #include "fa2_learn.cuh"
@@ -132,10 +133,12 @@ __device__ __forceinline__ bool learn_keep(float dq, float wx, float wy, float e
 // writes each body's repulsion in sorted order instead of the tail: the MLP
 // and k_learn_tail finish the iteration.  The sums are the same.
 //
+// AHEAD: walk_group's; go_traverse chooses.
+//
 // OVERLAP (prevent_overlap, with the monopole walk) repels accepted bodies by
 // the paper's anti-collision rule (overlap_factor) with the sizes of the
 // sorted bodies in ssize; a body node's sorted index is its owner's.
-template <bool QUAD, bool LEARN, bool OVERLAP, bool NORMAL_EPS>
+template <bool QUAD, bool LEARN, bool OVERLAP, bool NORMAL_EPS, bool AHEAD>
 __global__ void __launch_bounds__(kTravThreads, kTravWarpsPerSm *kWarp / kTravThreads) k_traverse(
     int n, const float4 *__restrict nodes, const float2 *__restrict quad,
     const uint32_t *__restrict body_node,
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__(kTravThreads, kTravWarpsPerSm *kWarp / kTravTh
         };
         // sum of m_j d / (d^2 + eps) over the accepted nodes; the body's own
         // k_r m_i multiplies the sum once at the end
-        const float2 a = walk_group<QUAD, OVERLAP, LEARN, NORMAL_EPS>(
+        const float2 a = walk_group<QUAD, OVERLAP, LEARN, NORMAL_EPS, AHEAD>(
             s_walk[wid], s_dq, nodes, quad, owner, ssize, end, px, py, my_size, prm.epssq,
             on_cells);
         // rounded on its own (never fused into the force sum that follows), so
@@ -787,21 +790,29 @@ void launch_place(const Buffers &b, const float2 *src_ref, int nblocks, cudaStre
 
 namespace {
 
-// At most one block per group: the blocks past that would find no work.
-int traverse_grid(const Buffers &b, int nblocks) { return std::min(nblocks, (b.n + 31) / 32); }
-
 template <bool QUAD, bool LEARN, bool OVERLAP>
 void go_traverse(const Buffers &b, const Params &p, const LearnBuffers &lb, int nblocks,
                  cudaStream_t s) {
+    const int groups = (b.n + 31) / 32;
+    // Loading ahead hides a round's load behind its test, for two more loads a
+    // lane.  While the SMs hold at most half of their warps the rounds' chain
+    // is what a walk waits for: 16.4 us without and 14.3 with it at 100 nodes,
+    // 28.6 and 24.6 at 5000, 36.9 and 34.6 at 40000, 43.4 and 42.9 at 75000.
+    // Above, the other warps fill the wait and the loads cost: 49.6 and 50.3
+    // at 90000, 252 and 271 on the scale-20 R-MAT layout.
+    const bool ahead = groups <= nblocks * (kTravThreads / kWarp) / 2;
     auto go = [&](auto kernel) {
-        kernel<<<traverse_grid(b, nblocks), kTravThreads, 0, s>>>(
+        // at most one block per group: the blocks past that would find no work
+        kernel<<<std::min(nblocks, groups), kTravThreads, 0, s>>>(
             b.n, b.nodes, b.quad, b.body_node, b.vals[0], b.fag, b.fprev, b.f, b.warp_partial,
             b.st, b.ctr, p, lb, b.owner, b.ssize);
     };
-    if (p.epssq >= FLT_MIN)
-        go(k_traverse<QUAD, LEARN, OVERLAP, true>);
-    else
-        go(k_traverse<QUAD, LEARN, OVERLAP, false>);
+    auto pick = [&](auto normal_eps) {
+        constexpr bool E = decltype(normal_eps)::value;
+        ahead ? go(k_traverse<QUAD, LEARN, OVERLAP, E, true>)
+              : go(k_traverse<QUAD, LEARN, OVERLAP, E, false>);
+    };
+    p.epssq >= FLT_MIN ? pick(std::true_type{}) : pick(std::false_type{});
 }
 
 }  // namespace

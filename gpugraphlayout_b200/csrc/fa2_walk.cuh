@@ -212,7 +212,11 @@ __device__ __forceinline__ bool walk_accepts(const Warp &W, float cx, float cy, 
 // body: 1e30, which passes every test) over the tree nodes[0 .. end).  Returns
 // the lane's sums.  `on_cells(accepted_cell, cell, thr, node)` is called once
 // per round by all lanes when ON_CELLS (the learned walk's pair list).
-template <bool QUAD, bool OVERLAP, bool ON_CELLS, bool NORMAL_EPS, class OnCells>
+//
+// AHEAD: a lane loads the two nodes that can follow its node, the first child
+// and the next one behind the subtree, beside the node's test, and has the
+// right one at hand in the next round.
+template <bool QUAD, bool OVERLAP, bool ON_CELLS, bool NORMAL_EPS, bool AHEAD, class OnCells>
 __device__ __forceinline__ float2 walk_group(WalkWarp<QUAD, OVERLAP> &W, const float (&dqs)[64],
                                              const float4 *nodes, const float2 *quad,
                                              const uint32_t *owner, const float *ssize,
@@ -229,6 +233,8 @@ __device__ __forceinline__ float2 walk_group(WalkWarp<QUAD, OVERLAP> &W, const f
     uint32_t node = 1, stop = lane == 0 ? end : 0u;
     int depth = 0;                 // stack entries
     uint32_t head = 0, tail = 0;   // list entries summed and held
+    float4 cur;  // AHEAD: the node's record, of a lane that holds one
+    if (AHEAD && node < stop) cur = nodes[node];
     for (;;) {
         bool idle = node >= stop;
         unsigned im = __ballot_sync(kFullMask, idle);
@@ -239,17 +245,23 @@ __device__ __forceinline__ float2 walk_group(WalkWarp<QUAD, OVERLAP> &W, const f
                 node = e.x;
                 stop = e.y;
                 idle = false;
+                if (AHEAD) cur = nodes[node];
             }
             depth = max(0, depth - __popc(im));
             im = __ballot_sync(kFullMask, idle);
         }
         if (im == kFullMask) break;
-        const float4 r = nodes[idle ? 0u : node];
+        const float4 r = AHEAD ? cur : nodes[idle ? 0u : node];
         const int meta = __float_as_int(r.w);
-        const int lvl = meta_level(meta);
+        const int lvl = idle ? kBodyLevel : meta_level(meta);
         const float thr = dqs[lvl];
-        const bool accept = walk_accepts(W, r.x, r.y, thr, eps) && !idle;
         const uint32_t next = meta_next(meta);
+        float4 behind, child;
+        if (AHEAD) {
+            behind = nodes[!idle && next < stop ? next : 0u];
+            child = nodes[lvl != kBodyLevel ? node + 1 : 0u];
+        }
+        const bool accept = walk_accepts(W, r.x, r.y, thr, eps) && !idle;
         // accepted nodes to the list
         const unsigned am = __ballot_sync(kFullMask, accept);
         if (accept) {
@@ -279,6 +291,7 @@ __device__ __forceinline__ float2 walk_group(WalkWarp<QUAD, OVERLAP> &W, const f
         }
         depth += __popc(pm);
         if (!idle) node = accept ? next : node + 1;
+        if (AHEAD) cur = accept ? behind : child;
         __syncwarp();
         if (tail - head >= (uint32_t)kWalkChunk) {
             walk_sum<QUAD, OVERLAP, NORMAL_EPS>(W, (int)(head & (kWalkList - 1)), kWalkChunk, px,

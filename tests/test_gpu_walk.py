@@ -61,3 +61,20 @@ def test_group_edges(n):
 def test_opening_angles(kind, theta):
     """From nearly every cell opened (full lists and stacks) to few."""
     _check(kind, 1201, theta)
+
+
+@pytest.mark.parametrize("n", [75776, 75777])
+def test_either_side_of_loading_ahead(n):
+    """Up to half of the resident warps (148 x 16 groups) a walk loads ahead."""
+    from gpugraphlayout_b200 import Engine
+    from oracle import oracle as O
+    s = np.arange(n, dtype=np.uint32)
+    g = O.Graph(s, np.roll(s, -1))
+    xy = _positions("uniform", n, 5)
+    e = Engine(g.n, g.sources, g.targets, scale=10.0)
+    e.set_positions(xy)
+    e.step(1)
+    tot, ga = e.forces()
+    ref, overflow, _ = O.Tree(xy, g.mass).repulsion(10.0)
+    assert not overflow
+    assert rel_rmse(tot - ga, np.asarray(ref).reshape(-1, 2)) <= TOL
