@@ -155,11 +155,6 @@ __device__ __forceinline__ bool deep_less(float2 pa, float2 pb, uint32_t ida, ui
     return ida < idb;
 }
 
-
-__device__ __forceinline__ int lcp_at(const uint64_t *__restrict keys, int n, int k) {
-    return (k < 0 || k >= n - 1) ? -1 : lcp_digits(keys[k], keys[k + 1]);
-}
-
 // cells that start at sorted body k
 __device__ __forceinline__ int cells_at(int k, int Lk, int Lkm1) {
     return k == 0 ? max(Lk, 0) + 1 : max(0, Lk - Lkm1);
@@ -206,57 +201,6 @@ __device__ __forceinline__ long long fixed_offset(float p, float root, double sc
     return __double2ll_rn(q);
 }
 
-
-__device__ __forceinline__ int load_lcp(const int8_t *__restrict lcp, int n, int k) {
-    return (k < 0 || k >= n - 1) ? -1 : (int)lcp[k];
-}
-
-// preorder index of sorted body b
-__device__ __forceinline__ uint32_t body_index(const int8_t *__restrict lcp,
-                                               const uint32_t *__restrict group, int n, int b) {
-    const int Lb = load_lcp(lcp, n, b), Lbm1 = load_lcp(lcp, n, b - 1);
-    return group[b] + (uint32_t)cells_at(b, Lb, Lbm1);
-}
-
-// Last body of the cell at level lvl that starts at sorted body k: the first
-// j >= k with L[j] < lvl.  Small cells end within a few bodies (a short scan
-// of L); larger ones are found by exponential + binary search over the keys
-// (LCP(K_k, K_j) falls as j grows).
-__device__ __forceinline__ int find_end(const uint64_t *__restrict keys, const int8_t *__restrict lcp, int n,
-                        int k, int lvl) {
-    constexpr int kScan = 8;
-    int L[kScan];
-#pragma unroll
-    for (int s = 0; s < kScan; ++s) L[s] = load_lcp(lcp, n, k + s);
-#pragma unroll
-    for (int s = 0; s < kScan; ++s)
-        if (L[s] < lvl) return k + s;
-    const uint64_t kk = keys[k];
-    int ok = k + kScan - 1, step = 1, bad = n;
-    for (;;) {
-        const int j = ok + step;
-        if (j >= n) {
-            bad = n;
-            break;
-        }
-        if (lcp_digits(keys[j], kk) >= lvl) {
-            ok = j;
-            step <<= 1;
-        } else {
-            bad = j;
-            break;
-        }
-    }
-    int lo = ok, hi = bad - 1;  // largest j with LCP(K_k, K_j) >= lvl, in [ok, bad)
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (lcp_digits(keys[mid], kk) >= lvl)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
 
 
 // The adaptive speed rule (SpeedKernel's last part, src/RPFA2Kernels.cu:177-219

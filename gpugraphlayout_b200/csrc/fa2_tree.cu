@@ -78,8 +78,7 @@ __device__ __forceinline__ Moments body_moments(longlong2 q, uint32_t m) {
 // The exclusive prefix of every sorted body's moments (pmom[k], and the total
 // at pmom[n]) in one pass: tiles of kMomTile bodies taken in ticket order,
 // each scanned in the block and offset by the tiles before it through a
-// decoupled look-back (the scheme of k_tree_count).  A wait that does not end
-// sets kErrScanWait.
+// decoupled look-back.  A wait that does not end sets kErrScanWait.
 __global__ void __launch_bounds__(kMomThreads) k_mom_scan(
     int n, const longlong2 *__restrict mq, const uint32_t *__restrict mm,
     MomLookback *__restrict lb, uint32_t *status, Moments *__restrict pmom, DevState *st,
