@@ -542,9 +542,9 @@ def run_ours(args, world, rank, local, fp64_n=FP64_CHECKS, correction=True):
         "config": workload_config(n, m, args.theta if learned is None else learned,
                                   args.multipole, args.workload, learned is not None),
         "clocks": clocks_summary(clk_path),
-        # + moment scan and per-cell a2 (quadrupole walk), + the cells'
-        # children moments, MLP and tail (learned correction)
-        "gpu_launches": (KERNELS_PER_ITER + (2 if args.multipole == 2 else 0)
+        # + per-cell a2 (quadrupole walk), + the cells' children moments, MLP
+        # and tail (learned correction)
+        "gpu_launches": (KERNELS_PER_ITER + (1 if args.multipole == 2 else 0)
                          + (3 if learned is not None else 0)) * args.steps,
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": 8 * n,
                 "d2h_bytes_per_step": 8 * n},

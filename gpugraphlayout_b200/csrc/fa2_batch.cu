@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(T, kBatchThreadsPerSm / T) k_batch(BatchArgs A
             // again, keeping gravity, attraction and the box of before.
             for (rounds = 0;; ++rounds) {
                 if (leader) ctl->ticket = 0;
-                build_tree(T_, team, B, A.chunk);
+                build_tree<T, false>(T_, team, B, A.chunk);
                 team.sync();
                 err = flag(&ctl->err);
                 if (err || !flag(&ctl->poison)) break;

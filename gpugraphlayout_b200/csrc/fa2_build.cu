@@ -51,6 +51,7 @@ struct GridTeam {
 
 // 64 registers and half an SM's threads per block: the attraction's blocks
 // share the SMs with it.
+template <bool MOM>
 __global__ void __launch_bounds__(kBuildThreads, 2) k_build(BuildArgs A, int chunk,
                                                             DevState *st, IterCounters *ctr) {
     extern __shared__ __align__(64) unsigned char smem_raw[];
@@ -67,12 +68,12 @@ __global__ void __launch_bounds__(kBuildThreads, 2) k_build(BuildArgs A, int chu
     // the pairs of the walk that follows (a learned iteration's)
     if (blockIdx.x == 0 && threadIdx.x < 16) ctr->pair_count[threadIdx.x] = 0;
     GridTeam team{(int)blockIdx.x, (int)gridDim.x, &ctr->build_bar, 0u, st};
-    build_tree(A, team, S, chunk);
+    build_tree<kBuildThreads, MOM>(A, team, S, chunk);
 }
 
 }  // namespace
 
-void launch_build(const Buffers &b, bool keep_moments, int nsm, cudaStream_t s) {
+void launch_build(const Buffers &b, bool moments, int nsm, cudaStream_t s) {
     BuildArgs A{};
     A.n = b.n;
     A.pos = b.pos;
@@ -94,8 +95,8 @@ void launch_build(const Buffers &b, bool keep_moments, int nsm, cudaStream_t s) 
     A.capacity = b.capacity;
     A.pm = b.pm;
     A.pxy = b.pxy;
-    A.mom_q = keep_moments ? b.mom_q : nullptr;
-    A.mom_m = keep_moments ? b.mom_m : nullptr;
+    A.pmom = b.pmom;
+    A.mom_totals = b.mom_totals;
     A.counts = b.sort_counts;
     A.hist = b.ctr->hist;
     A.totals = static_cast<NodeSums *>(b.build_totals);
@@ -119,12 +120,16 @@ void launch_build(const Buffers &b, bool keep_moments, int nsm, cudaStream_t s) 
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_build, A, chunk, b.st, b.ctr);
+    if (moments)
+        cudaLaunchKernelEx(&cfg, k_build<true>, A, chunk, b.st, b.ctr);
+    else
+        cudaLaunchKernelEx(&cfg, k_build<false>, A, chunk, b.st, b.ctr);
 }
 
 void build_set_smem_attr() {
-    cudaFuncSetAttribute(k_build, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)build_smem_bytes<kBuildThreads>(kBuildThreads * kBuildRounds));
+    const int most = (int)build_smem_bytes<kBuildThreads>(kBuildThreads * kBuildRounds);
+    cudaFuncSetAttribute(k_build<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    cudaFuncSetAttribute(k_build<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
 }
 
 size_t build_totals_bytes(int blocks) { return (size_t)blocks * sizeof(NodeSums); }

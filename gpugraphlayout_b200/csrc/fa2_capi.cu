@@ -138,9 +138,7 @@ int ensure_quad_buffers(fa2_ctx *c) {
     int s = FA2_OK;
     if ((!b.quad && (s = dalloc(c, &b.quad, b.capacity))) ||
         (!b.pmom && (s = dalloc(c, &b.pmom, (size_t)b.n + 1))) ||
-        (!b.mom_lb && (s = dalloc(c, &b.mom_lb, (size_t)mom_tiles(b.n)))) ||
-        (!b.mom_m && (s = dalloc(c, &b.mom_m, (size_t)b.n))) ||
-        (!b.mom_q && (s = dalloc(c, &b.mom_q, (size_t)b.n))))
+        (!b.mom_totals && (s = dalloc(c, &b.mom_totals, (size_t)build_blocks(b.n, c->nsm)))))
         return s;
     return FA2_OK;
 }
@@ -294,7 +292,7 @@ void enqueue_iteration(fa2_ctx *c, bool full, bool perturb_first, bool timed) {
             cudaEventRecordWithFlags(c->slot_events[slot * 2 + end], s, cudaEventRecordExternal);
     };
     const bool learn = c->learn_on;
-    // the moment scan and per-cell second moments of the quadrupole walk
+    // with the cells' second moments for the quadrupole walk
     const bool quad = c->kp.multipole >= 2;
     const bool side = full && c->overlap;  // stream B carries the attraction
     // A whole iteration finds its counters at zero (clear_counters) and leaves
@@ -316,13 +314,6 @@ void enqueue_iteration(fa2_ctx *c, bool full, bool perturb_first, bool timed) {
     mark(S_TREE, 0, A);
     launch_build(b, quad, c->nsm, A);
     mark(S_TREE, 1, A);
-    // the build leaves the sorted bodies' grid offsets and masses for the
-    // moment scan
-    if (quad) {
-        mark(S_MOM, 0, A);
-        launch_moments(b, A);
-        mark(S_MOM, 1, A);
-    }
     if (learn) {
         // the cells' second moments (a feature of the pairs), beside the walk
         // on stream B when it is in use; the MLP waits for them
@@ -331,10 +322,9 @@ void enqueue_iteration(fa2_ctx *c, bool full, bool perturb_first, bool timed) {
             cudaEventRecord(c->evEmitted, A);
             cudaStreamWaitEvent(B, c->evEmitted, 0);
         }
-        // timed in the moments slot, which the monopole walk leaves free
-        if (!quad) mark(S_MOM, 0, M);
+        mark(S_MOM, 0, M);
         launch_cell_a2(b, c->lb, c->nsm, M);
-        if (!quad) mark(S_MOM, 1, M);
+        mark(S_MOM, 1, M);
         if (side) cudaEventRecord(c->evA2, B);
     }
     if (side) cudaStreamWaitEvent(A, c->evJoin, 0);
@@ -867,14 +857,11 @@ fa2_ctx *fa2_create(const fa2_graph_desc *g, const fa2_params *prm, int *status)
     b.csr_w4 = d_w;
     b.ref_of = d_ref;
     b.build_totals = totals;
-    // one memset clears the counters and the moment scan's look-back flags
-    const size_t mom_status = (size_t)mom_tiles((int)n);
-    c->scratch_bytes = sizeof(IterCounters) + 4 * mom_status;
+    c->scratch_bytes = sizeof(IterCounters);
     char *scr = nullptr;
     if ((s = dalloc(c, &scr, c->scratch_bytes))) return fail(s);
     c->scratch = scr;
     b.ctr = (IterCounters *)scr;
-    b.mom_status = (uint32_t *)(scr + sizeof(IterCounters));
 
     // The tree chain (stream A) is the critical path; the attraction (stream B)
     // only has to finish before the traversal.  With A at the higher priority
@@ -1482,7 +1469,6 @@ int fa2_learn_collect(fa2_learn_set *set, fa2_ctx *c, float theta, int32_t multi
     c->seen_ok = false;
     CK(cudaMemsetAsync(set->st_count, 0, sizeof(unsigned long long), A));
     launch_build(b, multipole >= 2, c->nsm, A);
-    if (multipole >= 2) launch_moments(b, A);
     if (multipole >= 2) launch_quad_cells(b, c->nsm, A);
     launch_cell_a2(b, c->lb, c->nsm, A);
     launch_traverse_learn(b, kp, c->lb, c->trav_blocks, A);

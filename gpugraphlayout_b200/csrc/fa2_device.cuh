@@ -170,6 +170,12 @@ __device__ __forceinline__ i128 shfl_up_i128(i128 v, int o) {
     return ((i128)hi2 << 64) | (i128)lo2;
 }
 
+__device__ __forceinline__ i128 shfl_i128(i128 v, int from) {
+    const unsigned long long lo = __shfl_sync(kFullMask, (unsigned long long)v, from);
+    const long long hi = __shfl_sync(kFullMask, (long long)(v >> 64), from);
+    return ((i128)hi << 64) | (i128)lo;
+}
+
 __device__ __forceinline__ i128 shfl_xor_i128(i128 v, int o) {
     const unsigned long long lo = (unsigned long long)v;
     const long long hi = (long long)(v >> 64);

@@ -61,8 +61,7 @@ struct IterCounters {
     unsigned trav_ticket;
     unsigned trav_done;
     unsigned disp_done;
-    unsigned mom_ticket;
-    unsigned pad[2];
+    unsigned pad[3];
     unsigned pair_count[16];  // (group, cell) pairs of a learned walk, per pair segment
     unsigned hist[kBuildBins];  // keys per bin of the tree build's bucket sort
 };
@@ -75,11 +74,6 @@ inline int build_blocks(int n, int nsm) {
 }
 // Digit counts of the sort passes: [8][blocks][256].
 inline size_t build_counts(int blocks) { return (size_t)8 * blocks * 256; }
-
-// Moment scan (quadrupole option): bodies per tile and tiles.
-constexpr int kMomThreads = 256;
-constexpr int kMomTile = kMomThreads * 4;
-inline int mom_tiles(int n) { return (n + kMomTile - 1) / kMomTile; }
 
 // Attraction work split: rows (nodes in degree-descending order) with the
 // same number of lanes per row form one contiguous bucket.
@@ -102,12 +96,6 @@ struct AttractPlan {
 // |q| <= 2^45 every sum stays below 2^123.
 struct Moments {
     __int128 x, y, re, im;
-};
-
-// Look-back sums of one moment tile: its own total and, once known, the
-// total of every body up to its end.
-struct MomLookback {
-    Moments agg, incl;
 };
 
 struct Buffers {
@@ -133,10 +121,7 @@ struct Buffers {
     uint32_t *owner;          // capacity: per node, sorted body k << 6 | cell offset (63: body)
     float2 *quad;             // capacity: per cell, complex 2nd moment about its centre of mass
     Moments *pmom;            // n + 1: exclusive prefix of the body moments (quadrupole only)
-    longlong2 *mom_q;         // n: sorted bodies' offsets on the 2^-44 grid (null: not kept)
-    uint32_t *mom_m;          // n: sorted bodies' masses
-    MomLookback *mom_lb;      // moment tiles: look-back sums
-    uint32_t *mom_status;     // [moment tiles]: look-back flags (in the cleared scratch)
+    Moments *mom_totals;      // [build blocks]: their bodies' moments (quadrupole only)
     float4 *nodes;            // capacity + 1: x, y, mass, meta
     uint32_t capacity;
     long long *pm;            // n + 1: exclusive prefix of mass over sorted bodies
@@ -170,7 +155,7 @@ constexpr int kDispThreads = 512;
 // ---------------------------------------------------------------- kernels --
 void launch_bbox(const Buffers &b, int nblocks, cudaStream_t s);
 // The quadtree of the current positions, one cooperative launch.
-void launch_build(const Buffers &b, bool keep_moments, int nsm, cudaStream_t s);
+void launch_build(const Buffers &b, bool moments, int nsm, cudaStream_t s);
 size_t build_totals_bytes(int blocks);
 void build_set_smem_attr();
 // Bytes padded for vector loads of 64.
@@ -182,7 +167,6 @@ inline size_t pad64(size_t x) { return (x + 63) & ~(size_t)63; }
 constexpr int kShallowLevel = 22;
 constexpr int kMidLevel = 26;
 void launch_runs(const Buffers &b, int perturb, int nsm, cudaStream_t s);
-void launch_moments(const Buffers &b, cudaStream_t s);
 void launch_quad_cells(const Buffers &b, int nsm, cudaStream_t s);
 void launch_traverse(const Buffers &b, const Params &p, int nblocks, cudaStream_t s);
 void launch_displace(const Buffers &b, int nsm, cudaStream_t s);

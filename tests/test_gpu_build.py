@@ -126,3 +126,21 @@ def test_one_call_of_many_iterations_equals_one_call_per_iteration(n):
         out.append(e.get_positions())
     assert np.array_equal(out[0], out[1])
     assert np.array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("n", [2, 33, 512, 513, 4737, 20000])
+def test_quadrupole_moments_at_tile_edges(n):
+    """The build's prefix sums of the second moments, through the walk that
+    uses them."""
+    from gpugraphlayout_b200 import Engine
+    from oracle import oracle as O
+    g = _graph(n)
+    e = Engine(g.n, g.sources, g.targets, scale=10.0, theta=1.5, multipole=2)
+    for seed in (1, 2):
+        xy = _uniform(n, seed)
+        e.set_positions(xy)
+        e.step(1)
+        tot, ga = e.forces()
+        ref, overflow, _ = O.Tree(xy, g.mass).repulsion(10.0, itolsq=1 / 1.5 ** 2, multipole=2)
+        assert not overflow
+        assert rel_rmse(tot - ga, ref) <= TOL
