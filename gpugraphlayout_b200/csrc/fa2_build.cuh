@@ -149,16 +149,15 @@ constexpr int kMinRows = 256;
 
 // The bucket sort: bins by the keys' top bits (12 with 512 threads, 11 with
 // 256), the fullest bin it takes, and the keys per thread of a team.  Two
-// moves and two barriers instead of four of each: the build of a 300-node
-// graph takes 19 us instead of 23, of 10^4 nodes 39 instead of 44, an
-// iteration of 46717 nodes 81 instead of 87 and of 10^5 nodes 109 to 138
-// instead of 116 to 144.  Placing a key reads its whole bin: with bins of
-// 128 bodies the two ways meet (46000 normal positions: 49.6 us both; with
-// 512 allowed, 10^5 of them take 96 us instead of 70).  At four keys per
-// thread a 1.7 10^5-node iteration takes 205 us instead of 181.  The last
-// tree's cells tell most crowded layouts beforehand; the others lose 4 us
-// (4000 bodies) to 25 us (10^5) in their first build.  One atomic per warp and
-// bin (match) costs every other layout 1 us.
+// moves and two barriers instead of four of each: 4 us less for the build of
+// 300 nodes (23 us with the passes) and of 10^4 (44), 5 to 7 us less for an
+// iteration of 46717 (87) to 10^5 nodes (117, learned 144).  Placing a key
+// reads its whole bin: with bins of 128 bodies the two ways meet (46000 normal
+// positions: 49.6 us both; with 512 allowed, 10^5 of them take 96 us instead
+// of 70).  At four keys per thread a 1.7 10^5-node iteration takes 205 us
+// instead of 181.  The last tree's cells tell most crowded layouts beforehand;
+// the others lose 4 us (4000 bodies) to 25 us (10^5) in their first build.  One
+// atomic per warp and bin (match) costs every other layout 1 us.
 constexpr int kBinsPerThread = 8;
 constexpr uint32_t kBinMax = 128;
 constexpr int kBucketKeys = 2;  // keys per thread of a team's bucket sort
@@ -851,8 +850,8 @@ __device__ __forceinline__ CountOut build_count(const BuildArgs &A, int r0, int 
 // orders their global memory accesses and returns false when it gave up.
 // `chunk` is the number of keys the shared memory stages.
 // MOM: also the prefix sums of the bodies' second moments (pmom), for the
-// quadrupole option: the build of 1.7 10^5 bodies takes 79 us instead of 69,
-// a scan of its own behind the build took 22 (an iteration: 172 and 180 us).
+// quadrupole option: 10 us of the build of 1.7 10^5 bodies, where a scan of its
+// own behind the build took 22 (an iteration: 172 and 180 us).
 template <int T, bool MOM, class Team>
 __device__ __forceinline__ void build_tree(const BuildArgs &A, Team &team, BuildSmem<T> &S,
                                            int chunk) {
