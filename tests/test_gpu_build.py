@@ -144,3 +144,20 @@ def test_quadrupole_moments_at_tile_edges(n):
         ref, overflow, _ = O.Tree(xy, g.mass).repulsion(10.0, itolsq=1 / 1.5 ** 2, multipole=2)
         assert not overflow
         assert rel_rmse(tot - ga, ref) <= TOL
+
+
+@pytest.mark.parametrize("n", [3, 511, 512, 513])
+def test_order_after_a_displacement(n):
+    """The root box that the displacement leaves, by one block (up to 512
+    bodies) and by more: the next step's order is the oracle's of the
+    positions then."""
+    from gpugraphlayout_b200 import Engine
+    from oracle import oracle as O
+    g = _graph(n)
+    e = Engine(g.n, g.sources, g.targets, scale=10.0)
+    e.set_positions(_uniform(n, 6))
+    for _ in range(3):
+        e.step(1)
+        xy = e.get_positions()
+        e.step(1)
+        assert np.array_equal(e.sort_order(), O.Tree(xy, g.mass).sort().astype(np.uint32))
