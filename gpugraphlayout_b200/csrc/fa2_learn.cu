@@ -551,23 +551,27 @@ __global__ void __launch_bounds__(kMlpThreads) k_learn_mlp(
         // the next tile's first MMA overwrites the columns just read
         tc_fence_before();
         if (PAIRS) {
-            // Rows of one group are adjacent (the walk writes a group's cells
-            // in runs): sum each run within the warp, one atomic per run.
+            // Sum each run of rows of one group within the warp, one atomic per
+            // run.  A group can have several runs among the 32 rows (warps
+            // append to a segment in turn), so a run ends at the next row of
+            // another group, not where the group's number stops to match.
             const uint32_t grp = row < rows ? in.pair.x : 0xFFFFFFFFu;
             float cx = use ? sig * (c * y0 - s * y1) : 0.0f;
             float cy = use ? sig * (s * y0 + c * y1) : 0.0f;
+            const uint32_t prev = __shfl_up_sync(kFull, grp, 1);
+            const bool head = lane == 0 || prev != grp;
+            const uint32_t later = __ballot_sync(kFull, head) >> lane >> 1;
+            const int end = later ? lane + __ffs(later) : 32;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const float ox = __shfl_down_sync(kFull, cx, o);
                 const float oy = __shfl_down_sync(kFull, cy, o);
-                const uint32_t og = __shfl_down_sync(kFull, grp, o);
-                if (lane + o < 32 && og == grp) {
+                if (lane + o < end) {
                     cx += ox;
                     cy += oy;
                 }
             }
-            const uint32_t prev = __shfl_up_sync(kFull, grp, 1);
-            if (grp != 0xFFFFFFFFu && (lane == 0 || prev != grp)) {
+            if (grp != 0xFFFFFFFFu && head) {
                 atomicAdd(&corr[grp].x, cx);
                 atomicAdd(&corr[grp].y, cy);
             }

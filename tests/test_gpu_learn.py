@@ -212,3 +212,32 @@ def test_any_mlp_keeps_the_layout_finite():
     assert np.isfinite(e.get_positions()).all()
     st = e.stats()
     assert st["device_error"] == 0 and st["learned_pairs"] > 0
+
+
+@pytest.mark.parametrize("n,theta", [(3000, 1.3), (20000, 1.5)])
+def test_each_pair_counts_once_however_the_list_came_out(n, theta):
+    """The walk's warps append their pairs to the list in any order, so the
+    same positions give another order in each run.  The correction of a group
+    is the sum of its pairs' terms all the same: only rounding differs, at most
+    2^-24 per addition of a few hundred terms that do not cancel by more than a
+    few hundred, and 2^-24 of the force that the correction is read from."""
+    from gpugraphlayout_b200 import Engine, FarFieldMLP, synth
+    from oracle import oracle as O
+    g = O.Graph(*synth.ba_edges(n, 3, seed=2))
+    xy = O.random_positions(g.n, 20000, 20000, 8)
+    mlp = FarFieldMLP(seed=6)
+    e = Engine(g.n, g.sources, g.targets, strong_gravity=True, scale=1e6, gravity=1e-3, theta=theta)
+
+    def repulsion():
+        e.set_positions(xy)
+        e.step(1)
+        tot, ga = e.forces()
+        return (tot - ga).astype(np.float64)
+
+    plain = repulsion()
+    e.set_learned_correction(mlp)
+    corr = [repulsion() - plain for _ in range(8)]
+    size = np.sqrt(np.mean(corr[0] ** 2))
+    noise = 1e-2 * size + 2.0 ** -22 * np.abs(plain).max(axis=1, keepdims=True)
+    for c in corr[1:]:
+        assert (np.abs(c - corr[0]) <= noise).all()
