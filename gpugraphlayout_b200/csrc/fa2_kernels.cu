@@ -208,14 +208,13 @@ __global__ void __launch_bounds__(kTravThreads, kTravWarpsPerSm *kWarp / kTravTh
         }
         // LEARN: a round's accepted cells that the group sees at a size ratio
         // h / d of at least kLearnMinRatio theta (d from the group's centroid)
-        // go to this warp's segment of the pair list, one atomic per round
+        // go to the group's segment of the pair list, one atomic per round
         auto on_cells = [&](bool cell, const float4 &r, float thr, uint32_t node) {
             const bool keep = cell && learn_keep(thr, gx - r.x, gy - r.y, prm.epssq);
             const unsigned km = __ballot_sync(kFull, keep);
             if (km == 0) return;
             const unsigned nk = (unsigned)__popc(km);
-            const uint32_t seg = (blockIdx.x * (kTravThreads / kWarp) + (uint32_t)wid) %
-                                 (uint32_t)kPairSegments;
+            const uint32_t seg = (uint32_t)w % (uint32_t)kPairSegments;
             uint32_t base = 0;
             if (lane == 0) base = atomicAdd(&ctr->pair_count[seg], nk);
             base = __shfl_sync(kFull, base, 0);

@@ -70,9 +70,10 @@ __host__ __device__ constexpr uint32_t operand_offset(uint32_t r, uint32_t k, ui
 }
 
 // The pair list is split into kPairSegments segments of seg_cap pairs, each
-// with its own counter (IterCounters::pair_count): a warp appends to the
-// segment of its warp index, so the warps' reservations spread over 16
-// counters instead of queueing on one.
+// with its own counter (IterCounters::pair_count): a group's pairs go to the
+// segment of its index, so the reservations spread over 16 counters instead of
+// queueing on one, and the segments fill evenly whatever warps walk the groups
+// (with few groups only the first warp of each block has one).
 constexpr int kPairSegments = 16;
 
 // What the walk of a learned iteration leaves for the MLP and the tail.

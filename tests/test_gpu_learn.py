@@ -214,6 +214,16 @@ def test_any_mlp_keeps_the_layout_finite():
     assert st["device_error"] == 0 and st["learned_pairs"] > 0
 
 
+def _ring(n, seed, **options):
+    """An engine on a ring of n nodes at random positions, and those."""
+    from gpugraphlayout_b200 import Engine
+    xy = np.random.default_rng(seed).uniform(-1e4, 1e4, (n, 2)).astype(np.float32)
+    ids = np.arange(n, dtype=np.uint32)
+    e = Engine(n, ids, np.roll(ids, -1), strong_gravity=True, **options)
+    e.set_positions(xy)
+    return e, xy
+
+
 @pytest.mark.parametrize("n,theta", [(3000, 1.3), (20000, 1.5)])
 def test_each_pair_counts_once_however_the_list_came_out(n, theta):
     """The walk's warps append their pairs to the list in any order, so the
@@ -221,12 +231,9 @@ def test_each_pair_counts_once_however_the_list_came_out(n, theta):
     is the sum of its pairs' terms all the same: only rounding differs, at most
     2^-24 per addition of a few hundred terms that do not cancel by more than a
     few hundred, and 2^-24 of the force that the correction is read from."""
-    from gpugraphlayout_b200 import Engine, FarFieldMLP, synth
-    from oracle import oracle as O
-    g = O.Graph(*synth.ba_edges(n, 3, seed=2))
-    xy = O.random_positions(g.n, 20000, 20000, 8)
+    from gpugraphlayout_b200 import FarFieldMLP
     mlp = FarFieldMLP(seed=6)
-    e = Engine(g.n, g.sources, g.targets, strong_gravity=True, scale=1e6, gravity=1e-3, theta=theta)
+    e, xy = _ring(n, 8, scale=1e6, gravity=1e-3, theta=theta)
 
     def repulsion():
         e.set_positions(xy)
@@ -241,3 +248,16 @@ def test_each_pair_counts_once_however_the_list_came_out(n, theta):
     noise = 1e-2 * size + 2.0 ** -22 * np.abs(plain).max(axis=1, keepdims=True)
     for c in corr[1:]:
         assert (np.abs(c - corr[0]) <= noise).all()
+
+
+@pytest.mark.parametrize("n,theta", [(40, 0.3), (9000, 0.6), (18000, 0.4), (40000, 0.5)])
+def test_small_opening_angles_fit_the_pair_list(n, theta):
+    """The list holds 32 pairs per body (and 65,536 more) whatever warps walk
+    the groups: graphs with fewer groups than the GPU has warps included."""
+    from gpugraphlayout_b200 import FarFieldMLP
+    e, _ = _ring(n, 8, scale=10.0, theta=theta)
+    e.set_learned_correction(FarFieldMLP(seed=6))
+    e.step(1)
+    st = e.stats()
+    assert st["device_error"] == 0
+    assert st["learned_pairs"] <= 32 * n  # far from the limit, each case
