@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kTravThreads, kTravWarpsPerSm *kWarp / kTravTh
     DevState *st, IterCounters *ctr, Params prm, LearnBuffers lb,
     const uint32_t *__restrict owner, const float *__restrict ssize) {
     __shared__ WalkWarp<QUAD, OVERLAP> s_walk[kTravThreads / kWarp];
+    __shared__ uint32_t s_pairs[LEARN ? kTravThreads / kWarp : 1][LEARN ? 64 : 1];
     __shared__ float s_dq[64];
     __shared__ bool s_last;
     __shared__ float s_red[2][kTravThreads / kWarp];
@@ -208,26 +209,47 @@ __global__ void __launch_bounds__(kTravThreads, kTravWarpsPerSm *kWarp / kTravTh
         }
         // LEARN: a round's accepted cells that the group sees at a size ratio
         // h / d of at least kLearnMinRatio theta (d from the group's centroid)
-        // go to the group's segment of the pair list, one atomic per round
+        // wait in shared memory; 32 at a time go to the group's segment of the
+        // pair list.  A reservation a round, for two or three pairs, made the
+        // walk wait on its counter: 319 us instead of 206 on the scale-20 R-MAT
+        // layout at theta 1.5 (the plain walk takes 199), 55 instead of 40 at
+        // 90210 nodes; and the MLP sums a group's pairs in fewer runs.
+        int held = 0;
+        auto write_pairs = [&](int count) {
+            const uint32_t seg = (uint32_t)w % (uint32_t)kPairSegments;
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&ctr->pair_count[seg], (unsigned)count);
+            base = __shfl_sync(kFull, base, 0);
+            if (lane < count && base + (uint32_t)lane < lb.seg_cap)
+                lb.pairs[(size_t)seg * lb.seg_cap + base + (uint32_t)lane] =
+                    make_uint2((uint32_t)w, s_pairs[LEARN ? wid : 0][lane]);
+            if (lane == 0 && base + (uint32_t)count > lb.seg_cap) atomicOr(&st->err, kErrPairs);
+        };
         auto on_cells = [&](bool cell, const float4 &r, float thr, uint32_t node) {
             const bool keep = cell && learn_keep(thr, gx - r.x, gy - r.y, prm.epssq);
             const unsigned km = __ballot_sync(kFull, keep);
             if (km == 0) return;
-            const unsigned nk = (unsigned)__popc(km);
-            const uint32_t seg = (uint32_t)w % (uint32_t)kPairSegments;
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(&ctr->pair_count[seg], nk);
-            base = __shfl_sync(kFull, base, 0);
-            const uint32_t idx = base + (uint32_t)__popc(km & ((1u << lane) - 1u));
-            if (keep && idx < lb.seg_cap)
-                lb.pairs[(size_t)seg * lb.seg_cap + idx] = make_uint2((uint32_t)w, node);
-            if (lane == 0 && base + nk > lb.seg_cap) atomicOr(&st->err, kErrPairs);
+            uint32_t *q = s_pairs[LEARN ? wid : 0];
+            if (keep) q[held + __popc(km & ((1u << lane) - 1u))] = node;
+            held += __popc(km);
+            __syncwarp();
+            if (held < 32) return;
+            write_pairs(32);
+            held -= 32;
+            const uint32_t rest = lane < held ? q[32 + lane] : 0u;
+            __syncwarp();
+            if (lane < held) q[lane] = rest;
+            __syncwarp();
         };
         // sum of m_j d / (d^2 + eps) over the accepted nodes; the body's own
         // k_r m_i multiplies the sum once at the end
         const float2 a = walk_group<QUAD, OVERLAP, LEARN, NORMAL_EPS, AHEAD>(
             s_walk[wid], s_dq, nodes, quad, owner, ssize, end, px, py, my_size, prm.epssq,
             on_cells);
+        if (LEARN && held) {
+            write_pairs(held);
+            __syncwarp();
+        }
         // rounded on its own (never fused into the force sum that follows), so
         // the learned iteration, which stores it, adds the same value
         const float kmi = prm.k_r * me.z;
