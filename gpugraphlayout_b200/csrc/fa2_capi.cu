@@ -983,7 +983,8 @@ int fa2_step_host(fa2_ctx *c, const float *xy_in, int32_t n_iters, float *xy_out
     if (st.err) return FA2_ERR_DEVICE_LIMIT;
     int completed = st.iters_done - before;
     if (completed == n_iters && !st.poison) {
-        c->counters_zero = true;
+        // no iterations: nothing ran that would have cleared them
+        if (n_iters > 0) c->counters_zero = true;
         choose_sort_passes(c, st);
         return FA2_OK;
     }

@@ -261,3 +261,33 @@ def test_small_opening_angles_fit_the_pair_list(n, theta):
     st = e.stats()
     assert st["device_error"] == 0
     assert st["learned_pairs"] <= 32 * n  # far from the limit, each case
+
+
+@pytest.mark.parametrize("coincident", [False, True])
+def test_a_collection_leaves_nothing_to_the_next_step(coincident):
+    """fa2_learn_collect walks without the passes that end an iteration (and,
+    with two bodies in one place, stops in the tree build).  A step_host call
+    of no iterations after it, then a step: the order and the forces of an
+    engine that never collected, bit for bit.  More groups than the walk's
+    first wave has warps; some in the build's second block."""
+    from gpugraphlayout_b200 import LearnSet
+    n = 1500 if coincident else 160_001
+    out = []
+    for collect in (True, False):
+        e, xy = _ring(n, 3, scale=10.0)
+        if collect:
+            if coincident:
+                there = xy.copy()
+                there[7] = there[1200]
+                e.set_positions(there)
+            ls = LearnSet(20_000_000)
+            got = ls.collect(e, 2.0, 1)
+            assert (got == 0) == coincident
+            e.step_host(None, 0, np.zeros((n, 2), np.float32))
+            if coincident:
+                e.set_positions(xy)
+        e.step(1)
+        assert e.stats()["device_error"] == 0
+        out.append((e.sort_order(), e.forces()[0], e.get_positions()))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
