@@ -22,7 +22,7 @@
 //   fix     the sort leaves out the low digits that the last tree's cells
 //           hardly needed (sort_plan); every run of keys equal in the sorted
 //           digits is then put in the order of the full key, stably, which is
-//           exactly the full sort's order.  A run longer than kMaxRun sorts
+//           exactly the full sort's order.  A run longer than kFixRun sorts
 //           again on every digit;
 //   count   L[k], the bodies' records in sorted order, and the sums of each
 //           tile: nodes (a body's cells plus itself), mass and mass x position
@@ -133,6 +133,16 @@ struct BuildArgs {
 // fix phase puts in order are short.  Measured on the scale-20 R-MAT layout
 // and 10^4- to 10^5-node graphs: 3 or 4 passes instead of 8.
 constexpr int kThinCell = 32;
+// The longest run the fix phase puts in order, and the keys it loads at a time.
+// A body looks through its whole run, so long runs cost more than the sort on
+// every digit that follows a longer one.  The build of positions that share
+// level-12 cells after a tree that had none (us; one key at a time up to 1024,
+// then 4 at a time up to 128, 256 and 512): one cell of 3000 bodies 182, 80, 80
+// and 80, of 6 10^5 920, 270, 270 and 270; cells of 500, 10^5 bodies in all,
+// 197, 128, 128 and 145; of 250 136, 132, 110 and 112; of 150, 6 10^5 in all,
+// 257, 328, 227 and 233.  Eight loads at a time: 0 to 4 % longer.
+constexpr int kFixRun = 256;
+constexpr int kFixLoads = 4;
 __device__ __forceinline__ int sort_plan(const volatile int *cells) {
 #pragma unroll
     for (int i = 0; i < 5; ++i)
@@ -227,12 +237,14 @@ __device__ __forceinline__ uint32_t scan256(uint32_t v, BuildSmem<T> &S) {
 
 // The fix phase of this block's tile: every key of a run of keys equal above
 // `low` bits goes to its place by (key, input position), the others keep
-// theirs.
+// theirs.  A run longer than kFixRun needs the sort on every digit: nearly all
+// of its keys see that from the keys kFixRun and half as many places away.
 template <int T>
 __device__ __forceinline__ void build_fix(const BuildArgs &A, int low, const uint64_t *kin,
                                           const uint32_t *vin, uint64_t *kout, uint32_t *vout,
                                           int t0, int t1) {
     const int n = A.n;
+    bool resort = false;
     for (int i = t0 + (int)threadIdx.x; i < t1; i += T) {
         const uint64_t key = kin[i];
         const uint32_t v = vin[i];
@@ -241,28 +253,46 @@ __device__ __forceinline__ void build_fix(const BuildArgs &A, int low, const uin
         const bool left = low > 0 && i > 0 && (kin[i - 1] >> low) == hk;
         const bool right = low > 0 && i + 1 < n && (kin[i + 1] >> low) == hk;
         if (left || right) {
-            int s = i, smaller = 0;
-            while (s > 0 && i - s <= kMaxRun) {
-                const uint64_t o = kin[s - 1];
-                if ((o >> low) != hk) break;
-                --s;
-                smaller += o <= key;
+            int s = i, e = i + 1, smaller = 0;
+            auto same = [&](int j) { return j >= 0 && j < n && (kin[j] >> low) == hk; };
+            bool over = same(i - kFixRun) || same(i + kFixRun) ||
+                        (same(i - kFixRun / 2) && same(i + kFixRun / 2));
+            bool down = left && !over, up = right && !over;
+            while (down) {
+                uint64_t o[kFixLoads];
+                const int j = s - 1;
+#pragma unroll
+                for (int u = 0; u < kFixLoads; ++u) o[u] = kin[max(j - u, 0)];
+#pragma unroll
+                for (int u = 0; u < kFixLoads; ++u) {
+                    down = down && j - u >= 0 && (o[u] >> low) == hk;
+                    s -= down;
+                    smaller += down && o[u] <= key;
+                }
             }
-            int e = i + 1;
-            while (e < n && e - s <= kMaxRun) {
-                const uint64_t o = kin[e];
-                if ((o >> low) != hk) break;
-                ++e;
-                smaller += o < key;
+            while (up) {
+                uint64_t o[kFixLoads];
+                const int j = e;
+#pragma unroll
+                for (int u = 0; u < kFixLoads; ++u) o[u] = kin[min(j + u, n - 1)];
+#pragma unroll
+                for (int u = 0; u < kFixLoads; ++u) {
+                    up = up && j + u < n && (o[u] >> low) == hk;
+                    e += up;
+                    smaller += up && o[u] < key;
+                }
             }
-            if (e - s > kMaxRun)
-                atomicExch(A.resort, 1);
+            over |= e - s > kFixRun;
+            if (over)
+                resort = true;
             else
                 to = s + smaller;
         }
         kout[to] = key;
         vout[to] = v;
     }
+    // one store per block, not one per key
+    if (__syncthreads_or(resort) && threadIdx.x == 0) *(volatile int *)A.resort = 1;
 }
 
 // Where each of a chunk's keys goes by the digit at `shift`, stably: at[r] for

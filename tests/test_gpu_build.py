@@ -161,3 +161,24 @@ def test_order_after_a_displacement(n):
         xy = e.get_positions()
         e.step(1)
         assert np.array_equal(e.sort_order(), O.Tree(xy, g.mass).sort().astype(np.uint32))
+
+
+@pytest.mark.parametrize("n,count", [(500, 255), (500, 256), (500, 257), (500, 480), (3000, 129),
+                                     (3000, 255), (3000, 256), (3000, 257), (3000, 600),
+                                     (3000, 1100)])
+def test_long_runs_are_sorted_again(n, count):
+    """After a tree of thin cells the sort leaves out the levels past 12.  A
+    level-12 cell of up to 256 bodies is put in order by the fix-up; one of
+    more sorts on every digit, which counts as one of perturb_rounds."""
+    from gpugraphlayout_b200 import Engine
+    g = _graph(n)
+    e = Engine(g.n, g.sources, g.targets, scale=10.0)
+    _check(e, _uniform(n, 1), g.mass, False)
+    xy = _uniform(n, 2)
+    at = np.random.default_rng(3).permutation(64 * 64)[:count]  # in (0, 0.5)^2, 2048 / 4096 wide
+    xy[2:2 + count, 0] = (at % 64 + 0.5) / 128
+    xy[2:2 + count, 1] = (at // 64 + 0.5) / 128
+    _check(e, xy, g.mass, False)
+    assert e.stats()["perturb_rounds"] == (count > 256)
+    _check(e, xy, g.mass, False)  # the plan knows the cell now
+    assert e.stats()["perturb_rounds"] == 0
