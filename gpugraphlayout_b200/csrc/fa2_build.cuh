@@ -136,13 +136,14 @@ constexpr int kThinCell = 32;
 // The longest run the fix phase puts in order, and the keys it loads at a time.
 // A body looks through its whole run, so long runs cost more than the sort on
 // every digit that follows a longer one.  The build of positions that share
-// level-12 cells after a tree that had none (us; one key at a time up to 1024,
-// then 4 at a time up to 128, 256 and 512): one cell of 3000 bodies 182, 80, 80
-// and 80, of 6 10^5 920, 270, 270 and 270; cells of 500, 10^5 bodies in all,
-// 197, 128, 128 and 145; of 250 136, 132, 110 and 112; of 150, 6 10^5 in all,
-// 257, 328, 227 and 233.  Eight loads at a time: 0 to 4 % longer.
+// level-12 cells after a tree that had none, one key at a time up to 1024 and
+// this way: one cell of 3000 bodies 182 and 85 us, of 10^5 382 and 194, of 6 10^5
+// 920 and 285; 10^5 bodies in cells of 500 197 and 134, of 250 136 and 116, of
+// 150 103 and 94.  A limit of 128 takes 40 % longer for cells of 150, one of 512
+// 15 % longer for cells of 500; eight loads at a time 0 to 4 %.
 constexpr int kFixRun = 256;
 constexpr int kFixLoads = 4;
+static_assert(kThinCell % kFixLoads == 0, "where build_fix looks for a long run");
 __device__ __forceinline__ int sort_plan(const volatile int *cells) {
 #pragma unroll
     for (int i = 0; i < 5; ++i)
@@ -238,7 +239,8 @@ __device__ __forceinline__ uint32_t scan256(uint32_t v, BuildSmem<T> &S) {
 // The fix phase of this block's tile: every key of a run of keys equal above
 // `low` bits goes to its place by (key, input position), the others keep
 // theirs.  A run longer than kFixRun needs the sort on every digit: nearly all
-// of its keys see that from the keys kFixRun and half as many places away.
+// of its keys see that from the keys kFixRun and half as many places away, and
+// read no further.
 template <int T>
 __device__ __forceinline__ void build_fix(const BuildArgs &A, int low, const uint64_t *kin,
                                           const uint32_t *vin, uint64_t *kout, uint32_t *vout,
@@ -254,10 +256,13 @@ __device__ __forceinline__ void build_fix(const BuildArgs &A, int low, const uin
         const bool right = low > 0 && i + 1 < n && (kin[i + 1] >> low) == hk;
         if (left || right) {
             int s = i, e = i + 1, smaller = 0;
+            bool over = false, down = left, up = right;
+            // a key that has seen kThinCell of its run looks for a long one
             auto same = [&](int j) { return j >= 0 && j < n && (kin[j] >> low) == hk; };
-            bool over = same(i - kFixRun) || same(i + kFixRun) ||
-                        (same(i - kFixRun / 2) && same(i + kFixRun / 2));
-            bool down = left && !over, up = right && !over;
+            auto is_long = [&]() {
+                return same(i - kFixRun) || same(i + kFixRun) ||
+                       (same(i - kFixRun / 2) && same(i + kFixRun / 2));
+            };
             while (down) {
                 uint64_t o[kFixLoads];
                 const int j = s - 1;
@@ -268,6 +273,10 @@ __device__ __forceinline__ void build_fix(const BuildArgs &A, int low, const uin
                     down = down && j - u >= 0 && (o[u] >> low) == hk;
                     s -= down;
                     smaller += down && o[u] <= key;
+                }
+                if (down && i - s == kThinCell && is_long()) {
+                    over = true;
+                    down = up = false;
                 }
             }
             while (up) {
@@ -280,6 +289,10 @@ __device__ __forceinline__ void build_fix(const BuildArgs &A, int low, const uin
                     up = up && j + u < n && (o[u] >> low) == hk;
                     e += up;
                     smaller += up && o[u] < key;
+                }
+                if (up && e - 1 - i == kThinCell && is_long()) {
+                    over = true;
+                    up = false;
                 }
             }
             over |= e - s > kFixRun;
