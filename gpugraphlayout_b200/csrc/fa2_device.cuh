@@ -236,14 +236,19 @@ __device__ __forceinline__ void speed_update(float swg, float etra, int n, float
 
 // End of a pass that wrote one (swing, traction) partial per group of 32
 // sorted bodies: the last block to finish sums the partials in a fixed order
-// (thread-strided, then the warp's lanes, then the block's warps) and applies
-// the speed rule (src/RPFA2Kernels.cu:177-219).  Every thread of the block
-// calls it; s_last and s_red are the caller's shared memory.
+// and applies the speed rule (src/RPFA2Kernels.cu:177-219).  The order is that
+// of kSpeedSums strided sums, each its own chain of additions, then 32 of them
+// as a warp's lanes, then those one after the other, whatever the block's size:
+// the sums' rounding does not change with it, and a thread's chains of loads
+// run side by side.  Every thread of the block calls it; s_last and s_red are
+// the caller's shared memory.
+constexpr int kSpeedSums = 1024;
 template <int THREADS>
 __device__ __forceinline__ void speed_finish(int n, const float2 *warp_partial, unsigned *done,
                                              DevState *st, bool &s_last,
-                                             float (&s_red)[2][THREADS / kWarp]) {
-    const int lane = threadIdx.x & 31;
+                                             float (&s_red)[2][kSpeedSums / kWarp]) {
+    constexpr int kSums = kSpeedSums / THREADS;  // per thread
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nwarps = (n + 31) >> 5;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -253,25 +258,37 @@ __device__ __forceinline__ void speed_finish(int n, const float2 *warp_partial, 
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    float sw = 0.0f, tr = 0.0f;
-    for (int w = threadIdx.x; w < nwarps; w += THREADS) {
-        float2 v = __ldcg(&warp_partial[w]);
-        sw += v.x;
-        tr += v.y;
+    float sw[kSums] = {}, tr[kSums] = {};
+#pragma unroll 4
+    for (int w = threadIdx.x; w < nwarps; w += kSpeedSums) {
+        float2 v[kSums];
+#pragma unroll
+        for (int q = 0; q < kSums; ++q) {
+            const int at = w + q * THREADS;
+            v[q] = at < nwarps ? __ldcg(&warp_partial[at]) : make_float2(0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int q = 0; q < kSums; ++q) {  // no term is negative: adding 0 changes nothing
+            sw[q] += v[q].x;
+            tr[q] += v[q].y;
+        }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sw += __shfl_xor_sync(kFullMask, sw, o);
-        tr += __shfl_xor_sync(kFullMask, tr, o);
-    }
-    if (lane == 0) {
-        s_red[0][threadIdx.x >> 5] = sw;
-        s_red[1][threadIdx.x >> 5] = tr;
+    for (int q = 0; q < kSums; ++q) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            sw[q] += __shfl_xor_sync(kFullMask, sw[q], o);
+            tr[q] += __shfl_xor_sync(kFullMask, tr[q], o);
+        }
+        if (lane == 0) {
+            s_red[0][q * (THREADS / kWarp) + wid] = sw[q];
+            s_red[1][q * (THREADS / kWarp) + wid] = tr[q];
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         float swg = 0.0f, etra = 0.0f;
-        for (int w = 0; w < THREADS / kWarp; ++w) {
+        for (int w = 0; w < kSpeedSums / kWarp; ++w) {
             swg += s_red[0][w];
             etra += s_red[1][w];
         }

@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kTravThreads, kTravWarpsPerSm *kWarp / kTravTh
     __shared__ uint32_t s_pairs[LEARN ? kTravThreads / kWarp : 1][LEARN ? 64 : 1];
     __shared__ float s_dq[64];
     __shared__ bool s_last;
-    __shared__ float s_red[2][kTravThreads / kWarp];
+    __shared__ float s_red[2][kSpeedSums / kWarp];
     if (st->err || st->poison) return;
     if (threadIdx.x == 0) {
         walk_thresholds(st->radius, prm, s_dq);

@@ -895,7 +895,7 @@ __global__ void __launch_bounds__(kTravThreads, 2048 / kTravThreads) k_learn_tai
     const float2 *__restrict rep, const float2 *__restrict corr, DevState *st,
     IterCounters *ctr, Params prm) {
     __shared__ bool s_last;
-    __shared__ float s_red[2][kTravThreads / kWarp];
+    __shared__ float s_red[2][kSpeedSums / kWarp];
     if (st->err || st->poison) return;
     const int lane = threadIdx.x & 31;
     const int nwarps = (n + 31) >> 5;
