@@ -316,9 +316,10 @@ __device__ __forceinline__ float displacement_factor(float2 fi, float2 fp, float
 // pos is indexed by the ids in vals; ref_of maps them to reference ids (null:
 // the ids are reference ids).  The root cell is (rx, ry, rr); err and poison
 // receive the kErrRunTooLong bit and the coincidence count.
-__device__ __forceinline__ void fix_run(int k, int n, const uint64_t *__restrict keys,
-                                        uint32_t *__restrict vals, float2 *__restrict pos,
-                                        const uint32_t *__restrict ref_of, float rx, float ry,
+// Plain pointers: in the tree build other blocks wrote keys and vals earlier in
+// the same kernel, so no load may go through the read-only path.
+__device__ __forceinline__ void fix_run(int k, int n, const uint64_t *keys, uint32_t *vals,
+                                        float2 *pos, const uint32_t *ref_of, float rx, float ry,
                                         float rr, int *err, int *poison, int perturb) {
     const uint64_t key = keys[k];
     int len = 2;
