@@ -685,13 +685,17 @@ int configure(fa2_batch *b, uint32_t split, int small_threads, int large_threads
         first += (uint32_t)m.size();
         c.args.num_graphs = (int)m.size();
         c.args.queue = b->queues + k;
-        c.args.L = make_layout(nmax, c.team);
-        c.args.chunk = build_chunk(build_tile((int)nmax, c.team), c.threads);
-        c.smem = c.threads == 256 ? batch_smem_bytes<256>(c.args.chunk)
-                                  : batch_smem_bytes<512>(c.args.chunk);
         int teams = 0;
-        const int s = launch_class(c, b->kp.linlog != 0, b->stream, &teams);
-        if (s) return s;
+        for (;; c.team /= 2) {
+            c.args.L = make_layout(nmax, c.team);
+            c.args.chunk = build_chunk(build_tile((int)nmax, c.team), c.threads);
+            c.smem = c.threads == 256 ? batch_smem_bytes<256>(c.args.chunk)
+                                      : batch_smem_bytes<512>(c.args.chunk);
+            const int s = launch_class(c, b->kp.linlog != 0, b->stream, &teams);
+            if (s) return s;
+            // a context with a share of the SMs may hold no cluster of a size
+            if (teams > 0 || c.team == 1) break;
+        }
         c.grid = std::max(1, std::min<int>(teams, (int)m.size()));
         const size_t need = c.args.L.bytes * (size_t)c.grid;
         if (need > c.slot_cap) {

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kBuildThreads, 2) k_build(BuildArgs A, int chu
 
 }  // namespace
 
-void launch_build(const Buffers &b, bool moments, int nsm, cudaStream_t s) {
+cudaError_t launch_build(const Buffers &b, bool moments, cudaStream_t s) {
     BuildArgs A{};
     A.n = b.n;
     A.pos = b.pos;
@@ -112,7 +112,7 @@ void launch_build(const Buffers &b, bool moments, int nsm, cudaStream_t s) {
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cudaLaunchConfig_t cfg{};
-    const int blocks = build_blocks(b.n, nsm);
+    const int blocks = b.build_blocks;
     const int chunk = build_chunk(build_tile(b.n, blocks), kBuildThreads);
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.dynamicSmemBytes = build_smem_bytes<kBuildThreads>(chunk);
@@ -120,10 +120,8 @@ void launch_build(const Buffers &b, bool moments, int nsm, cudaStream_t s) {
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (moments)
-        cudaLaunchKernelEx(&cfg, k_build<true>, A, chunk, b.st, b.ctr);
-    else
-        cudaLaunchKernelEx(&cfg, k_build<false>, A, chunk, b.st, b.ctr);
+    return moments ? cudaLaunchKernelEx(&cfg, k_build<true>, A, chunk, b.st, b.ctr)
+                   : cudaLaunchKernelEx(&cfg, k_build<false>, A, chunk, b.st, b.ctr);
 }
 
 void build_set_smem_attr() {

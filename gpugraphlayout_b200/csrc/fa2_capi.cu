@@ -312,7 +312,7 @@ void enqueue_iteration(fa2_ctx *c, bool full, bool perturb_first, bool timed) {
     }
     if (perturb_first) launch_runs(b, 1, c->nsm, A);
     mark(S_TREE, 0, A);
-    launch_build(b, quad, c->nsm, A);
+    launch_build(b, quad, A);  // an error shows in the capture or the last error
     mark(S_TREE, 1, A);
     if (learn) {
         // the cells' second moments (a feature of the pairs), beside the walk
@@ -892,7 +892,13 @@ fa2_ctx *fa2_create(const fa2_graph_desc *g, const fa2_params *prm, int *status)
         cudaMemsetAsync(b.pos, 0, (size_t)n * 8, A) || cudaMemsetAsync(b.fprev, 0, (size_t)n * 8, A) ||
         cudaMemsetAsync(b.f, 0, (size_t)n * 8, A) || cudaMemsetAsync(b.fag, 0, (size_t)n * 8, A) ||
         cudaMemsetAsync(c->scratch, 0, c->scratch_bytes, A) ||
-        cudaMemsetAsync(b.st, 0, sizeof(DevState), A))
+        cudaMemsetAsync(b.st, 0xFF, sizeof(DevState), A))  // an error bit: the next launch does nothing
+        return fail(FA2_ERR_CUDA);
+    b.build_blocks = build_blocks((int)n, c->nsm);
+    if (launch_fitting(b.build_blocks, [&](int blocks) {
+            b.build_blocks = blocks;
+            return launch_build(b, false, A);
+        }) != cudaSuccess)
         return fail(FA2_ERR_CUDA);
     DevState st0;
     memset(&st0, 0, sizeof(st0));
@@ -1469,7 +1475,7 @@ int fa2_learn_collect(fa2_learn_set *set, fa2_ctx *c, float theta, int32_t multi
     if ((s = clear_counters(c))) return s;
     c->seen_ok = false;
     CK(cudaMemsetAsync(set->st_count, 0, sizeof(unsigned long long), A));
-    launch_build(b, multipole >= 2, c->nsm, A);
+    CK(launch_build(b, multipole >= 2, A));
     if (multipole >= 2) launch_quad_cells(b, c->nsm, A);
     launch_cell_a2(b, c->lb, c->nsm, A);
     launch_traverse_learn(b, kp, c->lb, c->trav_blocks, A);

@@ -66,11 +66,24 @@ struct IterCounters {
     unsigned hist[kBuildBins];  // keys per bin of the tree build's bucket sort
 };
 
-// Blocks of the tree build: 512 bodies or more each, at most one per SM.
+// Blocks of the tree build: 512 bodies or more each, at most one per SM; fewer
+// where the context holds fewer (Buffers::build_blocks).
 constexpr int kBuildMinTile = 512;
 inline int build_blocks(int n, int nsm) {
     const int b = (n + kBuildMinTile - 1) / kBuildMinTile;
     return b < 1 ? 1 : (b > nsm ? nsm : b);
+}
+// A cooperative grid has to be resident as a whole, and a context can hold less
+// than the device (an MPS client's share of the SMs): launch(blocks) with half
+// as many blocks until they fit, which a launch says before anything runs.
+template <class Launch>
+cudaError_t launch_fitting(int &blocks, Launch launch) {
+    for (;;) {
+        const cudaError_t e = launch(blocks);
+        if (e != cudaErrorCooperativeLaunchTooLarge || blocks <= 1) return e;
+        cudaGetLastError();  // refused, not failed
+        blocks = (blocks + 1) / 2;
+    }
 }
 // Digit counts of the sort passes: [8][blocks][256].
 inline size_t build_counts(int blocks) { return (size_t)8 * blocks * 256; }
@@ -126,6 +139,7 @@ struct Buffers {
     uint32_t capacity;
     long long *pm;            // n + 1: exclusive prefix of mass over sorted bodies
     __int128 *pxy;            // 2(n + 1): prefix of mass x fixed-point offset, x and y
+    int build_blocks;         // blocks of the tree build, at most build_blocks(n, SMs)
     void *build_totals;       // tree-build blocks: their tiles' sums (NodeSums)
     // reductions
     float4 *bbox_partial;     // bbox blocks
@@ -154,8 +168,9 @@ constexpr int kDispThreads = 512;
 
 // ---------------------------------------------------------------- kernels --
 void launch_bbox(const Buffers &b, int nblocks, cudaStream_t s);
-// The quadtree of the current positions, one cooperative launch.
-void launch_build(const Buffers &b, bool moments, int nsm, cudaStream_t s);
+// The quadtree of the current positions, one cooperative launch of
+// b.build_blocks blocks.  With an error bit set it returns at once.
+cudaError_t launch_build(const Buffers &b, bool moments, cudaStream_t s);
 size_t build_totals_bytes(int blocks);
 void build_set_smem_attr();
 // Bytes padded for vector loads of 64.

@@ -182,7 +182,12 @@ int run(const float *d_xy, const float *d_mass, uint32_t n, const fa2_params *pr
     const bool slot_was_clear = cudaPeekAtLastError() == cudaSuccess;
     k_prepare<<<(n + 255) / 256, 256, 0, s>>>(n, d_mass, const_cast<uint32_t *>(b.ref_of), b.fag, b.st);
     launch_bbox(b, d.nsm * 2, s);
-    launch_build(b, false, d.nsm, s);
+    b.build_blocks = build_blocks((int)n, d.nsm);
+    e = launch_fitting(b.build_blocks, [&](int blocks) {
+        b.build_blocks = blocks;
+        return launch_build(b, false, s);
+    });
+    if (e != cudaSuccess) return status_of(e);
     launch_traverse(b, kp, d.trav_blocks, s);
     if (slot_was_clear) {
         e = cudaGetLastError();
