@@ -791,7 +791,6 @@ fa2_batch *fa2_batch_create(uint32_t num_graphs, const fa2_graph_desc *graphs,
     }
     if (!(prm->theta > 0.0f)) return nullptr;
     uint64_t total_n = 0, total_m = 0;
-    uint32_t nmax = 1;
     for (uint32_t g = 0; g < num_graphs; ++g) {
         const fa2_graph_desc &d = graphs[g];
         if (d.num_edges && (!d.sources || !d.targets)) return nullptr;
@@ -810,7 +809,6 @@ fa2_batch *fa2_batch_create(uint32_t num_graphs, const fa2_graph_desc *graphs,
         }
         total_n += d.num_nodes;
         total_m += d.num_edges;
-        nmax = std::max(nmax, d.num_nodes);
     }
     if (total_n >= (1ull << 31) || 2 * total_m >= (1ull << 32)) {
         *status = FA2_ERR_TOO_LARGE;
@@ -891,7 +889,6 @@ fa2_batch *fa2_batch_create(uint32_t num_graphs, const fa2_graph_desc *graphs,
         return (uint64_t)graphs[a].num_nodes + graphs[a].num_edges >
                (uint64_t)graphs[c].num_nodes + graphs[c].num_edges;
     });
-    (void)nmax;
 
     BatchArgs &A = b->args;
 
@@ -937,7 +934,7 @@ fa2_batch *fa2_batch_create(uint32_t num_graphs, const fa2_graph_desc *graphs,
         cudaMemsetAsync(A.f_tot, 0, N * 8, st) || cudaMemsetAsync(A.f_ag, 0, N * 8, st) ||
         cudaMemsetAsync(A.sortd, 0, N * 4, st) || cudaStreamSynchronize(st))
         return fail(FA2_ERR_CUDA);
-    // every graph on 1024-thread CTAs until fa2_batch_configure / _autotune
+    // every graph on teams by its size until fa2_batch_configure / _autotune
     if ((s = configure(b, 0, 256, 1024))) return fail(s);
     *status = FA2_OK;
     return b;
@@ -1054,27 +1051,21 @@ int fa2_batch_autotune(fa2_batch *b, int32_t iters, uint32_t *split_out, int32_t
                 return FA2_ERR_CUDA;
         return cudaStreamSynchronize(b->stream) == cudaSuccess ? FA2_OK : FA2_ERR_CUDA;
     };
-    // candidates: the large graphs on 1024- or 512-thread CTAs, with every
-    // graph in that class or the graphs up to a size on smaller CTAs beside
+    // candidates, each with classes of its own (512 and 1024 are the same
+    // teams): every graph on teams by size, the graphs up to a size apart from
+    // the others on one 256-thread block or teams of their own, or every graph
+    // on one 256-thread block
     struct Cand {
         uint32_t split;
         int small, large;
-        bool operator==(const Cand &o) const {
-            return split == o.split && small == o.small && large == o.large;
-        }
     };
     uint32_t nmax = 1;
     for (uint32_t c : b->count) nmax = std::max(nmax, c);
-    std::vector<Cand> cand;
-    for (int large : {1024, 512}) {
-        cand.push_back(Cand{0u, 256, large});
-        for (uint32_t sp : {256u, 1024u, 4096u})
-            for (int t : {256, 512})
-                if (sp < nmax && t < large) cand.push_back(Cand{sp, t, large});
-    }
-    for (int t : {256, 512})
-        if (std::find(cand.begin(), cand.end(), Cand{nmax, t, 1024}) == cand.end())
-            cand.push_back(Cand{nmax, t, 1024});
+    std::vector<Cand> cand{Cand{0u, 256, 1024}};
+    for (uint32_t sp : {256u, 1024u, 4096u})
+        for (int t : {256, 512})
+            if (sp < nmax) cand.push_back(Cand{sp, t, 1024});
+    cand.push_back(Cand{nmax, 256, 1024});
     const Cand start{b->split, b->small_threads, b->large_threads};
     float best_ms = 0.0f;
     Cand best = start;

@@ -417,10 +417,9 @@ int fa2_batch_get_config(fa2_batch *batch, uint32_t *split, int32_t *small_threa
                          int32_t *large_threads);
 
 /* Picks the configuration by measurement: times `iters` iterations of every
- * candidate on this batch (large_threads 1024 or 512; no split, or graphs up
- * to 256, 1024 or 4096 nodes with 256 or 512; or all graphs with the small
- * setting), keeps the fastest, and puts the layout state
- * (positions, speeds, and the forces and orders of the last iteration) back
+ * candidate on this batch (large_threads 1024, which 512 equals; no split, or
+ * graphs up to 256, 1024 or 4096 nodes with small_threads 256 or 512; or all
+ * graphs with 256), keeps the fastest, and puts the layout state (positions, speeds, and the forces and orders of the last iteration) back
  * as it was.  Returns the choice and its ms per iteration. */
 int fa2_batch_autotune(fa2_batch *batch, int32_t iters, uint32_t *split,
                        int32_t *small_threads, int32_t *large_threads, float *ms_per_iter);

@@ -171,3 +171,16 @@ def test_autotune_leaves_the_layout_state_as_it_was():
     assert np.array_equal(b.get_positions(), ref.get_positions())
     with pytest.raises(Fa2Error):
         b.configure(100, 128, 1024)
+
+
+def test_autotune_times_no_classes_twice():
+    """512 and 1024 threads are the same teams: the choice between them is not
+    left to the noise of two trials of one configuration."""
+    graphs = _graphs([50, 700, 120])
+    b = _batch(graphs, scale=2.0)
+    b.set_positions(np.concatenate(_positions(graphs)))
+    picks = [b.autotune(1) for _ in range(16)]
+    assert {p["large_threads"] for p in picks} == {1024}
+    # every graph on teams is split 0, not a split at the largest graph
+    largest = max(g.n for g in graphs)
+    assert {p["small_threads"] for p in picks if p["split"] == largest} <= {256}
