@@ -182,3 +182,72 @@ def test_long_runs_are_sorted_again(n, count):
     assert e.stats()["perturb_rounds"] == (count > 256)
     _check(e, xy, g.mass, False)  # the plan knows the cell now
     assert e.stats()["perturb_rounds"] == 0
+
+
+def _cell_counts(xy, levels):
+    """Bodies in the fullest cell of each level under the box [-1024, 1024]^2."""
+    out = []
+    for lvl in levels:
+        c = np.ceil((xy.astype(np.float64) + 1024) * (2.0 ** lvl / 2048)).astype(np.int64)
+        out.append(int(np.unique(c, axis=0, return_counts=True)[1].max()))
+    return out
+
+
+def _nested(n, level, low, seed):
+    """More than 128 bodies in one level-6 cell (no bucket sort next time), 40
+    of them in one cell of `level`, apart four levels down; and 60 bodies in
+    one cell of the last level that a sort without its `low` lowest digits
+    tells apart."""
+    xy = _crowd(n, 200, seed, "spread")
+    rng = np.random.default_rng(seed)
+    w = 2048.0 / 2 ** level
+    at = rng.permutation(49)[:40]
+    xy[202:242, 0] = (at % 7 + 0.5) * (w / 7)
+    xy[202:242, 1] = (at // 7 + 0.5) * (w / 7)
+    if low:
+        w = 2048.0 / 2 ** (32 - 4 * low)
+        at = rng.permutation(64)[:60]
+        xy[242:302, 0] = -(at % 8 + 0.5) * (w / 8)
+        xy[242:302, 1] = -(at // 8 + 0.5) * (w / 8)
+    return xy
+
+
+# one block's sort in shared memory, and a team's through global memory
+@pytest.mark.parametrize("n", [500, 3000])
+@pytest.mark.parametrize("low", [5, 4, 3, 2, 1, 0])
+def test_order_with_each_number_of_digits_left_out(n, low):
+    """The sort leaves out the digits below the first of the levels 12, 16, ..,
+    28 at which the last tree's cells hold at most 32 bodies: every number of
+    moves, odd ones from the other buffer, and a run for the fix-up."""
+    from gpugraphlayout_b200 import Engine
+    g = _graph(n)
+    e = Engine(g.n, g.sources, g.targets, scale=10.0)
+    level = 28 - 4 * low
+    xy = _nested(n, level, 0, 1)
+    counts = _cell_counts(xy, [6, 12, 16, 20, 24, 28])
+    assert counts[0] > 128
+    assert next((5 - i for i in range(5) if counts[1 + i] <= 32), 0) == low
+    _check(e, xy, g.mass, False)
+    xy = _nested(n, level, low, 2)
+    if low:
+        assert _cell_counts(xy, [32 - 4 * low])[0] >= 60
+    _check(e, xy, g.mass, False)
+    assert e.stats()["perturb_rounds"] == 0
+
+
+@pytest.mark.parametrize("threads", [None, 256])
+@pytest.mark.parametrize("n", [1500, 2048, 2304])
+def test_batch_order_when_a_block_sorts_again(n, threads):
+    """A batch graph's first iteration knows no tree: 1100 bodies in one
+    level-24 cell are a run too long for the fix-up of the block's own sort."""
+    from gpugraphlayout_b200 import BatchEngine
+    from oracle import oracle as O
+    g = _graph(n)
+    b = BatchEngine([(g.n, g.sources, g.targets)], scale=10.0)
+    if threads:
+        b.configure(0, threads, threads)
+    xy = _crowd(n, 1100, 4, "tight")
+    assert _cell_counts(xy, [24])[0] > 1024
+    b.set_positions(xy)
+    b.step(1)
+    assert np.array_equal(b.sort_order(), O.Tree(xy, g.mass).sort().astype(np.uint32))
