@@ -11,8 +11,9 @@
 // working set stays in L2 across its iterations.  A team's scratch is one
 // slot, sized for the largest graph of its class.
 //
-// Why clusters: with one block per graph the batch took as long as its
-// largest graph, 1.7 ms for 20,000 nodes, while the other SMs ran dry.
+// Why clusters: with one block per graph a batch takes as long as its largest
+// graph (3.4 ms for 512 graphs of up to 20,000 nodes, 1.2 with clusters) while
+// the other SMs run dry.
 //
 // The reference has no batched mode: it lays out one graph per process, with
 // its speed and tree state in device statics (src/RPFA2Kernels.cu:29-33,
@@ -323,10 +324,10 @@ __device__ void phase_displace(const BatchArgs &A, const ClusterTeam &team, uint
 }
 
 // 1024 threads per SM, 64 registers a thread: a warp's walk has 32 loads in
-// flight, so it needs few warps, and at 32 registers it spills.  Measured on 512
-// graphs of 50 to 20,000 nodes (512-thread CTAs up to 4096 nodes, 1024-thread
-// CTAs above), 1024, 1536 and 2048 threads per SM: 1.74, 1.74 and 1.99 ms an
-// iteration; on 96 graphs of 50 to 600 nodes 90, 103 and 112 us.
+// flight, so it needs few warps, and at 32 registers it spills.  Measured with
+// 1024, 1536 and 2048 threads per SM: 512 graphs of 50 to 20,000 nodes 0.99, 0.98
+// and 1.12 ms an iteration (one 256-thread block each 4.18, 5.13 and 5.99), 96
+// graphs of 50 to 600 nodes 63, 72 and 80 us.
 constexpr int kBatchThreadsPerSm = 1024;
 
 // Launched in clusters of the team's size.
@@ -520,15 +521,29 @@ struct BatchClass {
 // A split's two sides, each of one class or one per team size.
 constexpr int kMaxClasses = 6;
 
-// How many 512-thread blocks (one cluster) run a graph of at most so many
-// nodes.  Measured on 512 graphs of 50 to 20,000 nodes: 1.16 ms an iteration;
-// teams of 4 already from 1024 nodes and of 8 from 4096 1.24 ms, of 4 only
-// from 4096 nodes 1.35 ms, of 2 instead of 4 1.28 ms.
-struct BatchTeam {
-    uint32_t upto;
-    int team;
-};
-constexpr BatchTeam kTeams[3] = {{2048, 1}, {8192, 4}, {kBatchMaxNodes, 8}};
+// How many 512-thread blocks (one cluster) run a graph: one up to `base` nodes,
+// four up to four times as many, eight above.  A cluster of four does the work of
+// about 2.8 blocks, so it is for graphs that would outlast the others: those of
+// more than half the nodes a resident block has on average, at least kTeamNodes.
+// A batch that one wave of single blocks holds, none of its graphs much above
+// that average, has none; where four blocks for every graph are resident at once
+// the line is kFewNodes.  Measured, ms an iteration, lines at 2048 / at the
+// average's half / at the average; 512, 1024 and 4096 graphs of 50 to 20,000
+// nodes: 1.19 / 1.19 / 1.34, 1.96 / 1.87 / 1.97, 7.94 / 6.74 / 6.74; 600 of 2500
+// nodes 1.01 / 0.83 / 0.83, 300 of 20,000 3.95 / 3.61 / 5.06, 296 of 4000 (one
+// wave) 0.71 / 0.71 / 0.56.  Lines at 2048 and 768: 8 of 2000 nodes 0.168 and
+// 0.067, 64 of 2000 0.170 and 0.089, of 1000 0.088 and 0.061, of 800 0.076 and
+// 0.057; 148 of 1500, more than fit at once, 0.131 and 0.193.
+constexpr uint32_t kTeamNodes = 2048, kFewNodes = 768;
+constexpr int kTeams[3] = {1, 4, 8};
+uint32_t team_base(uint64_t total_nodes, uint32_t graphs, uint32_t largest, int nsm) {
+    const uint64_t blocks = (uint64_t)nsm * (kBatchThreadsPerSm / 512);
+    if (graphs <= blocks && 3ull * largest * blocks <= 4 * total_nodes)
+        return std::max(largest, kTeamNodes);
+    const uint64_t least = 4ull * graphs <= blocks ? kFewNodes : kTeamNodes;
+    return (uint32_t)std::min<uint64_t>(std::max(total_nodes / (2 * blocks), least),
+                                        kBatchMaxNodes);
+}
 
 struct fa2_batch {
     int device = 0;
@@ -547,7 +562,7 @@ struct fa2_batch {
     // Graphs of at most `split` nodes run on `small_threads`, the others on
     // `large_threads`: 256 is one block of 256 threads per graph, 512 and 1024
     // are blocks of 512 threads, one or a cluster of them by the graph's size
-    // (kTeams).  The classes that makes, small graphs first.
+    // and the batch's (team_base).  The classes that makes, small graphs first.
     uint32_t split = 0;
     int small_threads = 256, large_threads = 1024;
     std::vector<BatchClass> cls;
@@ -648,10 +663,14 @@ int configure(fa2_batch *b, uint32_t split, int small_threads, int large_threads
         int threads, team;
     };
     std::vector<Kind> kinds;
+    uint32_t largest = 0;
+    for (uint32_t n : b->count) largest = std::max(largest, n);
+    const uint32_t base = team_base(b->total_nodes, b->num_graphs, largest, b->nsm);
     auto add = [&](uint32_t upto, int threads) {
         if (threads > 256)
-            for (const BatchTeam &k : kTeams)
-                kinds.push_back(Kind{std::min(upto, k.upto), 512, k.team});
+            for (int team : kTeams)
+                kinds.push_back(Kind{team == 8 ? upto : std::min(upto, base * (uint32_t)team), 512,
+                                     team});
         else
             kinds.push_back(Kind{upto, 256, 1});
     };

@@ -251,3 +251,40 @@ def test_batch_order_when_a_block_sorts_again(n, threads):
     b.set_positions(xy)
     b.step(1)
     assert np.array_equal(b.sort_order(), O.Tree(xy, g.mass).sort().astype(np.uint32))
+
+
+@pytest.mark.parametrize("n", [2049, 4608, 4609, 6001])
+def test_batch_order_when_single_blocks_fill_the_gpu(n):
+    """As many graphs as fill the GPU with one 512-thread block each: more
+    nodes than a cluster's line, either side of what a block's sort stages."""
+    from gpugraphlayout_b200 import BatchEngine
+    from oracle import oracle as O
+    g = _graph(n)
+    k = 224
+    b = BatchEngine([(g.n, g.sources, g.targets)] * k, scale=10.0)
+    xys = [_uniform(n, s) if s % 2 else _crowd(n, n // 8, s, "spread") for s in range(k)]
+    b.set_positions(np.concatenate(xys))
+    b.step(1)
+    order = b.sort_order()
+    tot, ga = b.forces()
+    for i in (0, 1, 112, 223):
+        t = O.Tree(xys[i], g.mass)
+        assert np.array_equal(b.part(order, i), t.sort().astype(np.uint32)), i
+        ref, overflow, _ = t.repulsion(10.0)
+        assert overflow or rel_rmse(b.part(tot - ga, i), ref) <= TOL, i
+
+
+def test_batch_order_of_a_few_small_graphs():
+    """Few enough graphs for four blocks each: the line lies at 768 nodes."""
+    from gpugraphlayout_b200 import BatchEngine
+    from oracle import oracle as O
+    sizes = [767, 768, 769, 1024, 3072, 3073]
+    graphs = [_graph(n) for n in sizes]
+    b = BatchEngine([(g.n, g.sources, g.targets) for g in graphs], scale=10.0)
+    for crowd in (False, True):
+        xys = [_crowd(n, 300, 5, "tight") if crowd else _uniform(n, 4) for n in sizes]
+        b.set_positions(np.concatenate(xys))
+        b.step(1)
+        order = b.sort_order()
+        for i, (g, xy) in enumerate(zip(graphs, xys)):
+            assert np.array_equal(b.part(order, i), O.Tree(xy, g.mass).sort().astype(np.uint32)), i
