@@ -47,7 +47,7 @@ RMAT = {"rmat20": (SCALE, DRAWS, WIDTH), "rmat23": (23, 134_217_728, 2.0e5)}
 FP64_SAMPLES = 4096
 FP64_EVERY, FP64_CHECKS = 50, 4
 # kernels per iteration: attract, tree build, traverse, displace; the quadrupole
-# walk adds the moment scan and the per-cell a2 kernel
+# walk adds the per-cell a2 kernel
 KERNELS_PER_ITER = 4
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_attract
 # launch at this workload, from an ncu capture of
@@ -619,6 +619,22 @@ def batch_cpu_baseline(graphs, sample_ids):
                       f"{total_n} nodes"}
 
 
+def batch_classes(sizes, cfg, nsm):
+    """Persistent launches of one batch step: a class per side of the split and
+    team size (team_base of csrc/fa2_batch.cu)."""
+    blocks, total, largest = 2 * nsm, sum(sizes), max(sizes, default=0)
+    if len(sizes) <= blocks and 3 * largest * blocks <= 4 * total:
+        base = max(largest, 2048)
+    else:
+        base = min(max(total // (2 * blocks), 768 if 4 * len(sizes) <= blocks else 2048), 65536)
+    found = set()
+    for n in sizes:
+        small = n <= cfg["split"]
+        one = cfg["small_threads" if small else "large_threads"] == 256
+        found.add((small, 0 if one else 1 if n <= base else 4 if n <= 4 * base else 8))
+    return len(found)
+
+
 def run_batched(args, world, rank, local):
     """The batched workload's record (rank 0; None on the other ranks)."""
     import torch
@@ -640,7 +656,8 @@ def run_batched(args, world, rank, local):
     eng.step_timed(args.steps)
     eng.step(1)
     sizes = [graphs[i][0] for i in mine]
-    classes = (any(s <= tuned["split"] for s in sizes) + any(s > tuned["split"] for s in sizes))
+    classes = batch_classes(sizes, tuned,
+                            torch.cuda.get_device_properties(local).multi_processor_count)
     clk_path = os.path.join(tempfile.gettempdir(), f"fa2_clocks_b{rank}.csv")
     sampler = clocks_sampler(local, clk_path)
     time.sleep(0.3)
@@ -694,7 +711,8 @@ def run_batched(args, world, rank, local):
                      "unit": "GB/s", "frac": achieved / hbm, "traffic": None,
                      "note": f"peak = {pk_kind} HBM copy bandwidth; achieved = compulsory bytes "
                              "of one iteration of every graph / time; the per-graph pipeline is "
-                             "latency-bound (one CTA per graph), so this is a lower bound"},
+                             "latency-bound (one team of CTAs per graph), so this is a lower "
+                             "bound"},
     }
     if world == 1 and not args.no_cpu_baseline:
         sizes = np.array([g[0] for g in graphs])

@@ -40,8 +40,15 @@ thread_local char g_last_cuda_error[192] = "";
 
 constexpr int kMaxReplayRounds = 64;
 // Iterations per captured graph of a longer step call: the gap between two
-// graphs is a few us, as long as a small graph's displacement.
+// graphs is a few us, as long as a small graph's displacement.  An iteration in
+// graphs of 1, 2, 4 and 8: 29.0, 27.8, 26.6 and 26.1 us at 100 nodes, 62.6, 61.3,
+// 60.5 and 59.5 at 10^4, 80.9, 74.7, 73.4 and 72.7 at 5 10^4.  The capture adds
+// 180 us to a new engine's first call (430 with 8), so 8 is not worth it.
 constexpr int kUnroll = 4;
+// Deepest tree levels after which a sort by depth would leave out its two lowest
+// digits (levels 24..31) or its lowest one (28..31): fa2_stats.sort_passes.
+constexpr int kShallowLevel = 22;
+constexpr int kMidLevel = 26;
 
 }  // namespace
 
@@ -82,6 +89,7 @@ struct fa2_ctx {
     std::vector<cudaEvent_t> event_pool;       // per (iteration, slot, start/end)
     int last_perturb_rounds = 0;
     int resorts_before = 0;  // DevState::resorts when the last step call began
+    int depth_passes = 8;    // fa2_stats.sort_passes
     bool overlap = true;  // attraction on stream B beside the tree build
     // accuracy guard (fa2_set_accuracy_guard)
     int guard_every = 0, guard_samples = 0, guard_cap = 0, guard_left = 0;
@@ -500,12 +508,11 @@ int resolve_poison(fa2_ctx *c, DevState *st) {
     return FA2_OK;
 }
 
-// The digits the last tree's depth lets the next sorts leave to the fix-up:
-// the two lowest after a tree no deeper than kShallowLevel, the lowest one
-// after one no deeper than kMidLevel (fa2_stats.sort_passes).
-void choose_sort_passes(fa2_ctx *c, const DevState &st) {
+// fa2_stats.sort_passes: the digits that the depth of the tree before calls for.
+// The sort itself goes by its cells' sizes (sort_plan).
+void note_depth_passes(fa2_ctx *c, const DevState &st) {
     const int l = st.max_level;
-    c->b.sort_first = l <= 0 ? 0 : (l <= kShallowLevel ? 2 : (l <= kMidLevel ? 1 : 0));
+    c->depth_passes = l <= 0 ? 8 : (l <= kShallowLevel ? 6 : (l <= kMidLevel ? 7 : 8));
 }
 
 // Runs n iterations; with `timed`, kernel_sum accumulates per-slot device ms.
@@ -519,7 +526,7 @@ int run_steps(fa2_ctx *c, int32_t n_iters, bool timed, std::vector<double> *kern
     c->last_perturb_rounds = 0;
     c->resorts_before = st.resorts;
     while (done < n_iters) {
-        choose_sort_passes(c, st);
+        note_depth_passes(c, st);
         // (re)captured here: a guard fallback drops the graphs
         if (timed && !c->exec_timed && (s = capture(c, true, 1, &c->exec_timed))) return s;
         const bool guard = guard_active(c);
@@ -991,7 +998,7 @@ int fa2_step_host(fa2_ctx *c, const float *xy_in, int32_t n_iters, float *xy_out
     if (completed == n_iters && !st.poison) {
         // no iterations: nothing ran that would have cleared them
         if (n_iters > 0) c->counters_zero = true;
-        choose_sort_passes(c, st);
+        note_depth_passes(c, st);
         return FA2_OK;
     }
     // An iteration needs a replay (coincident bodies): the iterations after it
@@ -1061,7 +1068,7 @@ int fa2_get_stats(fa2_ctx *c, fa2_stats *out) {
     out->root_y = st.rooty;
     out->interactions = st.interactions;
     out->visits = st.visits;
-    out->sort_passes = 8 - c->b.sort_first;
+    out->sort_passes = c->depth_passes;
     if (c->learn_on && c->n) {
         unsigned counts[kPairSegments];
         CK(cudaMemcpyAsync(counts, c->b.ctr->pair_count, sizeof(counts), cudaMemcpyDeviceToHost,

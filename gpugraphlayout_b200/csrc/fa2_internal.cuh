@@ -24,7 +24,7 @@ constexpr int kDeepLevels = 64;    // levels past 32 used to order such a run
 
 // Device error bits (DevState::err).  Any of them stops the iteration.
 enum : int {
-    kErrScanWait = 2,      // a block of the tree build or the moment scan waited too long
+    kErrScanWait = 2,      // a block of the tree build waited too long
     kErrRunTooLong = 4,    // more than kMaxRun bodies share a 64-bit key
     kErrTreeTooLarge = 8,  // the quadtree needs more nodes than allocated
     kErrNonFinite = 16,    // a position is NaN or infinite
@@ -67,7 +67,10 @@ struct IterCounters {
 };
 
 // Blocks of the tree build: 512 bodies or more each, at most one per SM; fewer
-// where the context holds fewer (Buffers::build_blocks).
+// where the context holds fewer (Buffers::build_blocks).  The build with 256, 512
+// and 1024 bodies as the least: 300 bodies 30.5, 18.0 and 18.3 us (one block needs
+// no barrier in global memory), 800 32.8, 32.8 and 24.1, 3000 34.4, 34.9 and 42.7,
+// 30000 37.7, 38.5 and 45.2.
 constexpr int kBuildMinTile = 512;
 inline int build_blocks(int n, int nsm) {
     const int b = (n + kBuildMinTile - 1) / kBuildMinTile;
@@ -146,7 +149,6 @@ struct Buffers {
     float2 *warp_partial;     // one per 32 sorted bodies
     DevState *st;
     IterCounters *ctr;
-    int sort_first;           // digits the last tree's depth lets the sort leave out (0, 1, 2)
     uint32_t *sort_counts;    // [8][tree-build blocks][256]: digit counts per tile and pass
     const float *size;        // n: node sizes for prevent_overlap (null: off)
     float *ssize;             // n: the same in sorted order, per iteration
@@ -175,12 +177,6 @@ size_t build_totals_bytes(int blocks);
 void build_set_smem_attr();
 // Bytes padded for vector loads of 64.
 inline size_t pad64(size_t x) { return (x + 63) & ~(size_t)63; }
-// Deepest tree levels after which the next sort may leave its two lowest
-// digits (levels 24..31) or its lowest one (levels 28..31) to the fix-up: bodies
-// then share at most that many digits, two levels short of those
-// (fa2_stats.sort_passes; the sort itself goes by the cells' sizes).
-constexpr int kShallowLevel = 22;
-constexpr int kMidLevel = 26;
 void launch_runs(const Buffers &b, int perturb, int nsm, cudaStream_t s);
 void launch_quad_cells(const Buffers &b, int nsm, cudaStream_t s);
 void launch_traverse(const Buffers &b, const Params &p, int nblocks, cudaStream_t s);

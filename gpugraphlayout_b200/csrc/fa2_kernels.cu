@@ -459,8 +459,8 @@ __global__ void __launch_bounds__(256) k_guard_finish(
     cur[s] = make_float2(f[i].x - fag[i].x, f[i].y - fag[i].y);
 }
 
-// One warp per sample: the plain walk of the sample's group (the k_traverse
-// loop at theta = 1); the sample's lane keeps its sum.
+// One warp per sample: the plain walk of the sample's group (the rule of
+// walk_group at theta = 1, one node at a time); the sample's lane keeps its sum.
 __global__ void __launch_bounds__(256) k_guard_plain(int n, int ns,
                                                      const float4 *__restrict nodes,
                                                      const uint32_t *__restrict body_node,
@@ -825,7 +825,11 @@ void go_traverse(const Buffers &b, const Params &p, const LearnBuffers &lb, int 
     // is what a walk waits for: 16.4 us without and 14.3 with it at 100 nodes,
     // 28.6 and 24.6 at 5000, 36.9 and 34.6 at 40000, 43.4 and 42.9 at 75000.
     // Above, the other warps fill the wait and the loads cost: 49.6 and 50.3
-    // at 90000, 252 and 271 on the scale-20 R-MAT layout.
+    // at 90000, 252 and 271 on the scale-20 R-MAT layout.  The other walks gain
+    // alike; at 1000, 20000 and 75000 nodes, without and with it: quadrupole 26.1
+    // and 24.0, 34.4 and 32.3, 48.6 and 46.6, learned 20.0 and 17.9, 26.1 and 24.0,
+    // 36.4 and 36.3, with node sizes 53.2 and 49.2, 79.7 and 73.7, 102.3 and 98.3;
+    // at 150000 they are within 2 us of each other.
     const bool ahead = groups <= nblocks * (kTravThreads / kWarp) / 2;
     auto go = [&](auto kernel) {
         // at most one block per group: the blocks past that would find no work

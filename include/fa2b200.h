@@ -136,7 +136,9 @@ int fa2_step_host(fa2_ctx *ctx, const float *xy_in, int32_t n_iters, float *xy_o
 int fa2_step_timed(fa2_ctx *ctx, int32_t n_iters, float *ms_total, float *kernel_ms,
                    int32_t n_kernels);
 
-/* Name of timed kernel slot i, or NULL past the last one. */
+/* Name of timed kernel slot i, or NULL past the last one.  The whole tree build
+ * is the slot "tree"; "keys", "sort", "tree_count" and "emit", its phases, keep
+ * their places and are always 0. */
 const char *fa2_kernel_name(int32_t i);
 
 /* Diagnostics of the last step; test and measurement hooks with no
@@ -158,14 +160,14 @@ typedef struct {
     float radius, root_x, root_y;
     uint64_t interactions;      /* body-node force terms of the last traversal */
     uint64_t visits;            /* body-node acceptance tests of the last traversal */
-    int32_t sort_passes;        /* 8-bit digit passes the last step's sorts take at most,
-                                   by the last tree's depth: 8; 6 after a tree no
-                                   deeper than level 22, 7 after one no deeper than 26.
-                                   The sort also leaves out low digits that the last
-                                   tree's cells hardly needed (runs of keys equal in
-                                   the sorted bits are then ordered by a fix-up, and a
-                                   run too long for it sorts again on every digit,
-                                   which counts as one of perturb_rounds) */
+    int32_t sort_passes;        /* 8-bit digits that the depth of the tree before the last
+                                   step calls for: 8; 6 after a tree no deeper than
+                                   level 22, 7 after one no deeper than 26.  A figure
+                                   of the depth, not a count of what the sort ran: that
+                                   goes by the cells' sizes, with buckets and no pass,
+                                   or 3 to 8 passes and a fix-up; bodies more crowded
+                                   than the tree before add 8 passes, which counts as
+                                   one of perturb_rounds */
     uint64_t learned_pairs;     /* (group, cell) pairs the last learned iteration's walk
                                    collected for the MLP (0 without the learned
                                    correction; see fa2_set_learned_correction) */
@@ -281,10 +283,9 @@ void fa2_mlp_init(fa2_mlp *mlp, uint32_t seed);
 
 /* Turns the correction on for the iterations that follow (mlp != NULL), on
  * top of the walk fa2_set_approximation selected (theta, multipole 1 or 2);
- * NULL turns it off.  The weights are copied.  A learned iteration also runs
- * the moment scan of the quadrupole option (the features need each cell's
- * second moment), the MLP and a separate tail kernel for the force sum and
- * the speed rule.  With all-zero weights it gives the plain walk's forces
+ * NULL turns it off.  The weights are copied.  A learned iteration also forms
+ * each cell's second moment from its children (a feature of the pairs) and runs
+ * the MLP and a separate tail kernel for the force sum and the speed rule.  With all-zero weights it gives the plain walk's forces
  * and positions bit for bit.  The accuracy guard (fa2_set_accuracy_guard)
  * checks the corrected repulsion and, on a fallback, also turns the
  * correction off. */
@@ -407,8 +408,8 @@ int fa2_batch_step_timed(fa2_batch *batch, int32_t n_iters, float *ms);
  * speed efficiency per graph. */
 /* CTA sizes: graphs of at most `split` nodes run with small_threads beside the
  * others with large_threads (each 256, 512 or 1024): 256 is one CTA of 256
- * threads per graph; 512 and 1024 are CTAs of 512 threads, one for a small
- * graph and a cluster of up to eight for a large one.  Each size class has its
+ * threads per graph; 512 and 1024 are CTAs of 512 threads, one or, for a graph
+ * that would outlast the others, a cluster of four or eight.  Each size class has its
  * own queue; the default is split 0 with 1024.  Results do not depend on the
  * choice, only the speed does. */
 int fa2_batch_configure(fa2_batch *batch, uint32_t split, int32_t small_threads,
