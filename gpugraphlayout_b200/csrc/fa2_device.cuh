@@ -258,37 +258,46 @@ __device__ __forceinline__ void speed_finish(int n, const float2 *warp_partial, 
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    float sw[kSums] = {}, tr[kSums] = {};
-#pragma unroll 4
-    for (int w = threadIdx.x; w < nwarps; w += kSpeedSums) {
-        float2 v[kSums];
-#pragma unroll
-        for (int q = 0; q < kSums; ++q) {
-            const int at = w + q * THREADS;
-            v[q] = at < nwarps ? __ldcg(&warp_partial[at]) : make_float2(0.0f, 0.0f);
-        }
-#pragma unroll
-        for (int q = 0; q < kSums; ++q) {  // no term is negative: adding 0 changes nothing
-            sw[q] += v[q].x;
-            tr[q] += v[q].y;
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < kSums; ++q) {
+    // of the 32 strided sums' warps, those that have a term
+    const int used = min((nwarps + 31) >> 5, kSpeedSums / kWarp);
+    auto warp_sum = [&](float a, float b, int at) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            sw[q] += __shfl_xor_sync(kFullMask, sw[q], o);
-            tr[q] += __shfl_xor_sync(kFullMask, tr[q], o);
+            a += __shfl_xor_sync(kFullMask, a, o);
+            b += __shfl_xor_sync(kFullMask, b, o);
         }
         if (lane == 0) {
-            s_red[0][q * (THREADS / kWarp) + wid] = sw[q];
-            s_red[1][q * (THREADS / kWarp) + wid] = tr[q];
+            s_red[0][at] = a;
+            s_red[1][at] = b;
         }
+    };
+    // no term is negative: adding 0 for one that is not there changes nothing
+    auto term = [&](int at) {
+        return at < nwarps ? __ldcg(&warp_partial[at]) : make_float2(0.0f, 0.0f);
+    };
+    if (nwarps <= THREADS) {  // one term a thread, without the other way's code
+        const float2 v = term(threadIdx.x);
+        warp_sum(v.x, v.y, wid);
+    } else {
+        float sw[kSums] = {}, tr[kSums] = {};
+#pragma unroll 4
+        for (int w = threadIdx.x; w < nwarps; w += kSpeedSums) {
+            float2 v[kSums];
+#pragma unroll
+            for (int q = 0; q < kSums; ++q) v[q] = term(w + q * THREADS);
+#pragma unroll
+            for (int q = 0; q < kSums; ++q) {
+                sw[q] += v[q].x;
+                tr[q] += v[q].y;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kSums; ++q) warp_sum(sw[q], tr[q], q * (THREADS / kWarp) + wid);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         float swg = 0.0f, etra = 0.0f;
-        for (int w = 0; w < kSpeedSums / kWarp; ++w) {
+        for (int w = 0; w < used; ++w) {
             swg += s_red[0][w];
             etra += s_red[1][w];
         }
