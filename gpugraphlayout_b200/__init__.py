@@ -325,8 +325,8 @@ class BatchEngine:
     def configure(self, split: int, small_threads: int = 256, large_threads: int = 1024) -> None:
         """Graphs of at most `split` nodes with small_threads, the rest with
         large_threads (split 0: all of them).  256: one CTA of 256 threads per
-        graph; 512 and 1024: CTAs of 512 threads, one for a small graph and a
-        cluster of up to eight for a large one."""
+        graph; 512 and 1024: CTAs of 512 threads, one or, for a graph that would
+        outlast the others, a cluster of four or eight."""
         check(lib().fa2_batch_configure(self._b, int(split), int(small_threads),
                                         int(large_threads)), "fa2_batch_configure")
 

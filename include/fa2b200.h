@@ -148,7 +148,8 @@ typedef struct {
     uint32_t tree_nodes;        /* cells + bodies of the last quadtree */
     uint32_t tree_cells;
     int32_t max_level;          /* deepest cell level (root 0) */
-    int32_t perturb_rounds;     /* .99 re-insertion rounds in the last step */
+    int32_t perturb_rounds;     /* .99 re-insertion rounds in the last step, and sorts
+                                   done again on every digit */
     int32_t device_error;       /* bit set of device-side limit hits, 0 = none:
                                    2 tree-build wait limit, 4 more than 1024 bodies on
                                    one 64-bit key, 8 tree larger than its buffer,
